@@ -12,6 +12,7 @@ the device from the seed; the shapes are the benchmark's (`bench.py`) and the te
     run(state)          one pass
     work(case)          bytes and operations a pass cannot do without
     tolerance(case)     how far another correct implementation may be from this one
+    exact(case, seed)   what a pass returns, evaluated in 64 bits by plain torch
 """
 from __future__ import annotations
 
@@ -141,12 +142,17 @@ def _run_mmvq(c, s):
     return ops.mmvq(s["w"], ops.TYPE_Q8_0, c["k"], c["n"], s["x"])
 
 
+def _inputs_ffn(c, gen):
+    hidden, inter = c["hidden"], c["inter"]
+    weights = [(_q4_k(gen, inter, hidden), _q4_k(gen, inter, hidden), _q4_k(gen, hidden, inter))
+               for _ in range(c["layers"])]
+    return weights, _normal(gen, c["layers"], c["tokens"], hidden)
+
+
 def _prepare_ffn(c, gen):
     hidden, inter, tokens = c["hidden"], c["inter"], c["tokens"]
     glu = ops.GLU_GEGLU if c["glu"] == "geglu" else ops.GLU_SWIGLU
-    weights = [(_q4_k(gen, inter, hidden), _q4_k(gen, inter, hidden), _q4_k(gen, hidden, inter))
-               for _ in range(c["layers"])]
-    x = _normal(gen, c["layers"], tokens, hidden)
+    weights, x = _inputs_ffn(c, gen)
     y = torch.empty_like(x)
     h = torch.empty((tokens, inter), device="cuda")
     q8x, q8h = ops.quantize_q8(x[0]), ops.quantize_q8(h.zero_())
@@ -162,10 +168,14 @@ def _prepare_ffn(c, gen):
     return {"weights": weights, "x": x, **_captured(step)}
 
 
+def _inputs_proj(c, gen):
+    weights = [_q8_0(gen, c["n"], c["k"]) for _ in range(c["layers"])]
+    return weights, _normal(gen, c["layers"], c["tokens"], c["k"])
+
+
 def _prepare_proj(c, gen):
     k, n, tokens = c["k"], c["n"], c["tokens"]
-    weights = [_q8_0(gen, n, k) for _ in range(c["layers"])]
-    x = _normal(gen, c["layers"], tokens, k)
+    weights, x = _inputs_proj(c, gen)
     y = torch.empty((c["layers"], tokens, n), device="cuda")
     q8 = ops.quantize_q8(x[0])
 
@@ -178,10 +188,9 @@ def _prepare_proj(c, gen):
     return {"weights": weights, "x": x, **_captured(step)}
 
 
-def _prepare_decode_vector(c, gen):
-    k, n, tokens = c["k"], c["n"], c["tokens"]
-    x = _normal(gen, c["layers"], tokens, k)
-    y = torch.empty((c["layers"], tokens, n), device="cuda")
+def _inputs_decode_vector(c, gen):
+    k, n = c["k"], c["n"]
+    x = _normal(gen, c["layers"], c["tokens"], k)
     weights = []
     for _ in range(c["layers"]):
         if c["decoder"] == "q8_0":
@@ -191,6 +200,13 @@ def _prepare_decode_vector(c, gen):
             weights.append((ops.DECODER_MXFP8_ATOMS, codes, atoms))
         else:
             weights.append((ops.DECODER_BF16, (_normal(gen, n, k) * 0.02).bfloat16().view(torch.uint8), None))
+    return weights, x
+
+
+def _prepare_decode_vector(c, gen):
+    k, n, tokens = c["k"], c["n"], c["tokens"]
+    weights, x = _inputs_decode_vector(c, gen)
+    y = torch.empty((c["layers"], tokens, n), device="cuda")
 
     def step():
         for i, (decoder, data, scales) in enumerate(weights):
@@ -200,10 +216,14 @@ def _prepare_decode_vector(c, gen):
     return {"weights": weights, "x": x, **_captured(step)}
 
 
-def _prepare_mmq(c, gen):
+def _inputs_mmq(c, gen):
     x = _normal(gen, c["tokens"], c["k"])
-    w = _q4_k(gen, c["n"], c["k"])
-    s = {"x": x.bfloat16() if c["bf16"] else x, "w": w, "slab": None}
+    return _q4_k(gen, c["n"], c["k"]), x.bfloat16() if c["bf16"] else x
+
+
+def _prepare_mmq(c, gen):
+    w, x = _inputs_mmq(c, gen)
+    s = {"x": x, "w": w, "slab": None}
     if c["slab"]:
         s["slab"], s["w"] = ops.q4k_relayout(w, c["k"], c["n"]), None
     return s
@@ -223,20 +243,26 @@ def _run_mxfp8(c, s):
     return ops.mxfp8_gemm(a, a_scales, s["w"], s["w_scales"], bf16=True)
 
 
-def _prepare_moe(c, gen):
+def _inputs_moe(c, gen):
+    """Per layer: activations, the experts' weights, and the router's choice for every token."""
     tokens, experts, used, hidden, inter = (c[n] for n in ("tokens", "experts", "used", "hidden", "inter"))
-    layers = []
     for _ in range(c["layers"]):
         gate_up = _q4_k(gen, experts * 2 * inter, hidden).view(experts, 2 * inter, -1)
         down = _q4_k(gen, experts * hidden, inter).view(experts, hidden, -1)
         p, ids = torch.topk(torch.softmax(_normal(gen, tokens, experts), 1), used, dim=1)
+        yield gate_up, down, ids.int(), (p / p.sum(1, keepdim=True)).contiguous(), _normal(gen, tokens, hidden)
+
+
+def _prepare_moe(c, gen):
+    tokens, hidden, inter = c["tokens"], c["hidden"], c["inter"]
+    layers = []
+    for gate_up, down, ids, weights, x in _inputs_moe(c, gen):
         # a prefill's experts as a program relays them at load time
         slabs = None
         if tokens >= MOE_PREFILL:
             slabs = (ops.q4k_relayout(gate_up, hidden, 2 * inter, glu=True),
                      ops.q4k_relayout(down, inter, hidden), True)
-        layers.append((_normal(gen, tokens, hidden), ids.int(), (p / p.sum(1, keepdim=True)).contiguous(),
-                       gate_up, down, slabs))
+        layers.append((x, ids, weights, gate_up, down, slabs))
 
     def step():
         return [ops.moe_ffn(x, ids, w, gate_up, down, hidden, inter, slabs=slabs)
@@ -306,3 +332,110 @@ def tolerance(case: dict) -> dict:
         return {"rel": 5e-3}            # results rounded to BF16
     # the intermediate is quantized to 8 bits: a sum in another order moves some of its codes
     return {"rel": 1e-3, "max": 0.05}
+
+
+# ------------------------------------------------------------------ the same in 64 bits
+# The block formats' own roundings (8-bit codes, FP16 scales and sums) are part of what a pass
+# returns and are restated; every product and sum is taken in 64 bits.
+def _f16(raw: torch.Tensor) -> torch.Tensor:
+    return raw.contiguous().view(torch.float16).squeeze(-1)
+
+
+def _blocks_of_32(x: torch.Tensor, reciprocal: bool):
+    """x F32 [rows, k] as 8-bit blocks: codes [rows, k / 32, 32], scales and sums [rows, k / 32]."""
+    v = x.float().view(x.shape[0], -1, 32)
+    amax = v.abs().amax(2, keepdim=True)
+    live = torch.where(amax > 0, amax, torch.ones_like(amax))
+    if reciprocal:
+        inverse = 127.0 / live
+        codes, d = (v * inverse).double(), 1.0 / inverse
+    else:
+        d = live / 127.0
+        codes = (v / d).double()
+    codes = torch.trunc(codes + torch.where(codes < 0, -0.5, 0.5))
+    d = torch.where(amax > 0, d, torch.zeros_like(d))
+    q = v.view(x.shape[0], v.shape[1], 8, 4)
+    p = ((q[..., 0] + q[..., 1]) + q[..., 2]) + q[..., 3]
+    s = ((p[..., 0] + p[..., 4]) + (p[..., 2] + p[..., 6])) + ((p[..., 1] + p[..., 5]) + (p[..., 3] + p[..., 7]))
+    return codes, d.squeeze(2).half().double(), s.half().double()
+
+
+def _q4_k_parts(w: torch.Tensor):
+    """Codes [rows, k / 32, 32], FP16 d and dmin [rows, k / 256, 1], scales and minima [rows, k / 256, 8]."""
+    b = w.reshape(w.shape[0], -1, 144)
+    d, dmin, s = _f16(b[:, :, 0:2])[..., None], _f16(b[:, :, 2:4])[..., None], b[:, :, 4:16].int()
+    sc = torch.cat([s[..., 0:4] & 63, (s[..., 8:12] & 15) | ((s[..., 0:4] >> 6) << 4)], 2)
+    mn = torch.cat([s[..., 4:8] & 63, (s[..., 8:12] >> 4) | ((s[..., 4:8] >> 6) << 4)], 2)
+    c = b[:, :, 16:].view(b.shape[0], b.shape[1], 4, 32)
+    return torch.stack([c & 15, c >> 4], 3).view(b.shape[0], -1, 32), d, dmin, sc, mn
+
+
+def _dot_q4_k(w: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
+    """The decode products' x [rows, k] by Q4_K rows: the minima multiply the codes' sums."""
+    codes, d, dmin, sc, mn = _q4_k_parts(w)
+    scale = (d.double() * sc).view(w.shape[0], -1, 1)
+    minimum = (dmin.double() * mn).view(w.shape[0], -1, 1)
+    dense = (codes.double() * scale - minimum).view(w.shape[0], -1)
+    q, d8, _ = _blocks_of_32(x, False)
+    return (q * d8[..., None]).view(x.shape[0], -1) @ dense.T
+
+
+def _matmul_q4_k(w: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
+    """The prefill products': FP16 products of the scales, the minima multiply the inputs' sums."""
+    codes, d, dmin, sc, mn = _q4_k_parts(w)
+    scale = (d * sc.half()).double().view(w.shape[0], -1, 1)
+    minimum = (dmin * mn.half()).double().view(w.shape[0], -1)
+    dense = (codes.double() * scale).view(w.shape[0], -1)
+    q, d8, s8 = _blocks_of_32(x, True)
+    return (q * d8[..., None]).view(x.shape[0], -1) @ dense.T - s8 @ minimum.T
+
+
+def _dot_q8_0(w: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
+    q, d8, _ = _blocks_of_32(x, False)
+    return (q * d8[..., None]).view(x.shape[0], -1) @ _dense_q8_0(w).T
+
+
+def _dense_q8_0(w: torch.Tensor) -> torch.Tensor:
+    b = w.view(w.shape[0], -1, 34)
+    return (_f16(b[:, :, 0:2]).double()[..., None] * b[:, :, 2:].contiguous().view(torch.int8)).view(w.shape[0], -1)
+
+
+def _glu(kind: str, gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
+    f = torch.nn.functional
+    return (f.gelu(gate, approximate="tanh") if kind == "geglu" else f.silu(gate)) * up
+
+
+def exact(case: dict, seed: int):
+    c, kind = case, case["kind"]
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(seed)
+    if kind == "mmvq":
+        s = _prepare_mmvq(c, gen)
+        return _dot_q8_0(s["w"], s["x"])
+    if kind == "ffn":
+        weights, x = _inputs_ffn(c, gen)
+        return torch.stack([_dot_q4_k(down, _glu(c["glu"], _dot_q4_k(gate, x[i]), _dot_q4_k(up, x[i])))
+                            for i, (gate, up, down) in enumerate(weights)])
+    if kind == "proj":
+        weights, x = _inputs_proj(c, gen)
+        return torch.stack([_dot_q8_0(w, x[i]) for i, w in enumerate(weights)])
+    if kind == "decode_vector" and c["decoder"] != "mxfp8":
+        weights, x = _inputs_decode_vector(c, gen)
+        return torch.stack([x[i].double() @ (_dense_q8_0(w) if c["decoder"] == "q8_0" else
+                                             w.view(torch.bfloat16).double()).T
+                            for i, (_, w, _) in enumerate(weights)])
+    if kind == "mmq":
+        return _matmul_q4_k(*_inputs_mmq(c, gen))
+    if kind == "moe":
+        outs = []
+        for gate_up, down, ids, weights, x in _inputs_moe(c, gen):
+            dot = _matmul_q4_k if c["tokens"] >= MOE_PREFILL else _dot_q4_k
+            y = torch.zeros(x.shape, dtype=torch.float64, device="cuda")
+            for e in ids.unique().tolist():
+                rows, slots = (ids == e).nonzero(as_tuple=True)
+                gu = dot(gate_up[e], x[rows])
+                h = _glu("swiglu", gu[:, :c["inter"]], gu[:, c["inter"]:])
+                y.index_add_(0, rows, dot(down[e], h) * weights[rows, slots, None].double())
+            outs.append(y)
+        return outs
+    return None  # MXFP8: the weights in hand are this package's own quantization of them
