@@ -347,10 +347,11 @@ def _blocks_of_32(x: torch.Tensor, reciprocal: bool):
     amax = v.abs().amax(2, keepdim=True)
     live = torch.where(amax > 0, amax, torch.ones_like(amax))
     if reciprocal:
-        inverse = 127.0 / live
-        codes, d = (v * inverse).double(), 1.0 / inverse
+        # (one rounding: a number over a tensor would be the reciprocal times the number)
+        inverse = torch.full_like(live, 127.0) / live
+        codes, d = (v * inverse).double(), torch.ones_like(live) / inverse
     else:
-        d = live / 127.0
+        d = live / torch.full_like(live, 127.0)
         codes = (v / d).double()
     codes = torch.trunc(codes + torch.where(codes < 0, -0.5, 0.5))
     d = torch.where(amax > 0, d, torch.zeros_like(d))
