@@ -9,43 +9,49 @@
 //
 // The int8 contraction runs on tcgen05 (kind::i8, int32 accumulators in TMEM).
 // Q4_K's per-group scales forbid accumulating across groups in the tensor
-// core, so every 128 x 128 x 32 MMA lands in its own TMEM buffer (three of them,
-// so the tensor core runs ahead) and a wide epilogue (16 warps) folds each
-// group's int32 tile into F32 register accumulators: acc += ((d*sc) * C) * d8.
-// The MMA's M side (the TMEM lanes) is the TOKENS and its N side (the TMEM
-// columns) the weight rows: an epilogue thread is one token with 32 weight rows
-// in registers, so the activation scale d8 is one scalar a thread and group,
-// the weight scales d*sc are one broadcast 128-bit shared load per four
-// elements, and a thread's results are 128 contiguous bytes of the output.
+// core, so every group's 128 x 128 x 32 product has to be read out of TMEM and
+// folded into F32 register accumulators, and that fold is what bounds the kernel.
+// The tensor core, idle for most of it, also forms the group's SCALE products:
+// d8 (per token) x (d*sc)_half (per weight row) is a rank-1 FP16 product (kind::f16, K
+// 16 of which one is not zero, F32 accumulate: 22 bits, exact), written beside the
+// integers, so the fold is two TMEM loads a piece, a conversion a value and one packed
+// multiply-add a pair: acc += C * (d8 * d*sc), one rounding.  (With the scales as
+// broadcast shared-memory loads, two packed instructions a pair and 16 warps of 32
+// rows: 139 warp instructions and 1,030 cycles a group; 2.5e-7 off the double product
+// where this is 2.1e-7.)
+// The MMA's M side (the TMEM lanes) is the TOKENS and its N side (the TMEM columns) the
+// weight rows: a thread's results are contiguous in the output.
 // The min terms need no integer product: sum over groups of (-dmin*m)_half *
 // s8_half is a plain FP16 contraction over K = k / 32, which the tensor core
-// takes (kind::f16, F32 accumulate, a fourth TMEM buffer) from two small K-major
-// FP16 tiles; the epilogue adds that buffer once at the end.
+// takes (kind::f16, F32 accumulate) from two small K-major FP16 tiles: every 64
+// groups it takes a TMEM buffer's turn, and the epilogue adds it.
 //
 // Weights reach the MMA in one of two ways.
 //   * SLAB (llmp_b200_q4k_relayout once at load time, or per call into caller
 //     scratch): the Q4_K blocks unpacked to what the tensor core reads, int8
 //     codes K-major, (d*sc)_half as F32 in [k-step][group][row] tiles, (-dmin*m)
-//     as FP16 K-major.  The producer warp brings all of it by TMA straight into
-//     the swizzled tiles; nothing is decoded in the GEMM's critical path.
+//     half K-major; the producer warp's TMA brings the codes and minima straight into
+//     the swizzled tiles.
 //   * RAW (no slab, no scratch): two decode warps unpack the Q4_K blocks of a
 //     TMA-fed raw stage into the same tiles, k-step by k-step.
+//
+// One persistent CTA an SM (all of its tensor memory): the next tile's operands and
+// first groups are on their way under a tile's write-back.
 //
 //   warp 0       TMA producer: per k-step the activation int8 tile (128 tokens x
 //                128 K bytes) straight out of the [k/128][col] block array through
 //                a 3-D tensor map (row pitch 144 B, origin past the 16-byte block
-//                header) and, with a slab, the weight tile and its scales; per
-//                two k-steps the tokens' block headers (and, raw, the weight
-//                rows' Q4_K blocks) into a raw stage;
-//   warps 1-2    the activation headers into d8 (F32) and s8 (FP16, the min
-//                tile); raw mode: also the weight blocks into the int8 tile, the
-//                four groups' d*sc and -dmin*m;
-//   warp 3       allocates TMEM and issues the MMAs;
-//   warps 4-19   epilogue: thread = (token, a quarter of the weight rows): loads
-//                its 32 columns, hands the buffer back to the tensor core at
-//                once, then folds.
+//                header) and, with a slab, the weight tile; per two k-steps the tokens'
+//                block headers and the weight rows' scales (raw: their Q4_K blocks) into
+//                a raw stage;
+//   warp 1       allocates TMEM and issues the MMAs;
+//   warps 2-3    the scale tiles (d8; d*sc) and s8 (the min tile) of a k-step; raw mode:
+//                also the weight blocks into the int8 tile and -dmin*m;
+//   warps 4-11   epilogue: thread = (token, half of the weight rows).
 // Rows past the matrix and tokens past the batch are TMA's zero fill.
 // Every wait is bounded; a wait that runs out raises the device fault counter.
+#include <algorithm>
+
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -238,32 +244,51 @@ constexpr int kTileCols = 128;  // tokens: the MMA's M, one TMEM lane each
 constexpr int kTileRows = 128;  // weight rows: the MMA's N, one TMEM column each
 constexpr int kBK = 128;        // K bytes a stage: four 32-value groups
 constexpr int kStages = 3;
-constexpr int kBuffers = 3;     // TMEM group-result buffers of kTileRows columns
-constexpr int kMinColumn = kBuffers * kTileRows;  // TMEM: the F32 sum of the min terms
+// A TMEM buffer holds a group's integer tile and, beside it, its scale tile; two of them are all
+// 512 columns, so the min terms' sum takes a buffer's turn instead of columns of its own.
+constexpr int kBuffers = 2;
+constexpr int kScaleColumn = kTileRows;
+constexpr int kBufferColumns = 2 * kTileRows;
 constexpr int kWBytes = kTileRows * kBK, kYBytes = kTileCols * kBK;
-constexpr int kScaleBytes = 4 * 128 * 4;  // [group][row or token] F32
-constexpr int kStageBytes = kWBytes + kYBytes + (2 * kScaleBytes);
+// The scale tile's operands, one pair a group: K 16 of which only k = 0 is not zero.  K-major
+// without swizzle: 8 rows x 16 bytes (k = 0..7) a core matrix, the groups of 8 rows 128 bytes
+// apart; k = 8..15 of every operand is one shared tile of zeros, reached by the leading offset.
+constexpr int kScaleTileBytes = 128 * 16;
+constexpr int kStageScaleBytes = 4 * kScaleTileBytes;  // [group]
+constexpr int kStageBytes = kWBytes + kYBytes + (2 * kStageScaleBytes);
 // The min terms' operands: FP16 [128 rows or tokens][64 groups] K-major, 128-byte
-// swizzled like the int8 tiles; one tile holds 16 k-steps, two tiles alternate.
+// swizzled like the int8 tiles; one tile holds 16 k-steps.  With a slab two tiles alternate,
+// raw blocks leave room for one.
 constexpr int kMinTileBytes = 128 * 128;
 constexpr int kMinSteps = 16;  // k-steps a tile of min operands covers
-// Raw stages: what TMA brings for one super-block column (two k-steps): the 128
-// weight rows' Q4_K blocks (raw mode only), then the 128 tokens' block headers of
-// both k-steps.
+template <bool kSlab>
+constexpr int kMinTiles = kSlab ? 2 : 1;
+// Raw stages: what TMA brings for one super-block column (two k-steps): the 128 weight rows'
+// Q4_K blocks, or with a slab the rows' scales of both k-steps; then the 128 tokens' block
+// headers of both.
 constexpr int kRawStages = 2;
-constexpr int kRawWBytes = 128 * 144;
+constexpr int kAxBytes = 4 * 128 * 4;  // a k-step's d * sc in a slab
+template <bool kSlab>
+constexpr int kRawWBytes = kSlab ? 2 * kAxBytes : 128 * 144;
 constexpr int kRawHBytes = 128 * 16;
-constexpr int kRawBytes = kRawWBytes + (2 * kRawHBytes);
-constexpr int kEpilogueWarps = 16;
-constexpr int kDecodeWarps = 2;  // warps 1 .. kDecodeWarps
-constexpr int kMmaWarp = kDecodeWarps + 1;
-constexpr int kFirstEpilogueWarp = kDecodeWarps + 2;  // a multiple of 4: warp % 4 is its TMEM quadrant
+template <bool kSlab>
+constexpr int kRawBytes = kRawWBytes<kSlab> + (2 * kRawHBytes);
+constexpr int kMmaWarp = 1;
+constexpr int kFirstDecodeWarp = 2;
+constexpr int kDecodeWarps = 2;  // a thread takes two weight rows and two tokens
+static_assert(kTileRows == kTileCols, "a row and a token an item");
+constexpr int kFirstEpilogueWarp = kFirstDecodeWarp + kDecodeWarps;
+// Eight epilogue warps of 64 weight rows a thread rather than 16 of 32: twelve warps leave 168
+// registers a thread, which hold the 64 sums and two 16-row pieces, so a piece's loads run under
+// the fold of the one before.
+constexpr int kEpilogueWarps = 8;
 constexpr int kThreads = (kFirstEpilogueWarp + kEpilogueWarps) * 32;
-static_assert(kFirstEpilogueWarp % 4 == 0, "epilogue warp e must sit in TMEM quadrant e % 4");
 constexpr int kEpilogueRows = kTileRows / (kEpilogueWarps / 4);  // weight rows a thread
-static_assert(kEpilogueRows == 32, "one 32-column TMEM load a group");
-constexpr int kSmem =
-    (kStages * kStageBytes) + (4 * kMinTileBytes) + (kRawStages * kRawBytes) + 1024 + 512;
+static_assert(kEpilogueRows == 64, "two 32-row groups a thread");
+template <bool kSlab>
+constexpr int kSmem = (kStages * kStageBytes) + (2 * kMinTiles<kSlab> * kMinTileBytes) +
+                      (kRawStages * kRawBytes<kSlab>) + kScaleTileBytes + 512;
+static_assert(kSmem<true> <= 232448 && kSmem<false> <= 232448, "a CTA's shared memory");
 
 // Two F32 lanes in one 64-bit register: sm_100's packed F32 arithmetic does two
 // roundings-to-nearest per instruction, the same results as two scalar ones.
@@ -275,9 +300,9 @@ __device__ __forceinline__ std::uint64_t Pack2(float lo, float hi) {
 __device__ __forceinline__ void Unpack2(std::uint64_t v, float& lo, float& hi) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
-__device__ __forceinline__ std::uint64_t Mul2(std::uint64_t a, std::uint64_t b) {
+__device__ __forceinline__ std::uint64_t Add2(std::uint64_t a, std::uint64_t b) {
   std::uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 __device__ __forceinline__ std::uint64_t Fma2(std::uint64_t a, std::uint64_t b, std::uint64_t c) {
@@ -289,14 +314,13 @@ __device__ __forceinline__ std::uint64_t Fma2(std::uint64_t a, std::uint64_t b, 
 struct Shared {
   std::uint64_t y_full[kStages];   // the stage's TMA bytes have landed
   std::uint64_t w_full[kStages];   // the decode warps have written their part
-  std::uint64_t empty[kStages];
+  std::uint64_t empty[kStages];    // the tensor core has read the stage
   std::uint64_t tmem_full[kBuffers];
   std::uint64_t tmem_empty[kBuffers];
   std::uint64_t raw_full[kRawStages];
   std::uint64_t raw_empty[kRawStages];
   std::uint64_t minw_full[2];  // slab mode: a tile of weight min operands has landed
   std::uint64_t min_free[2];   // the tensor core has read a tile of min operands
-  std::uint64_t min_full;      // the min terms' sum is complete in tensor memory
   std::uint32_t tmem_base;
   std::uint32_t abort;
 };
@@ -308,7 +332,8 @@ struct Params {
   const float* ax;       // slab: the scale tiles
   int ax_ksteps;         // k-steps a row tile's scales span
   int ax_row_tiles;
-  std::int32_t* sums;    // verification: the int32 group sums [col][row][k / 32], or null
+  int col_tiles;         // of an expert, or the worklist's capacity
+  std::int32_t* sums;    // verification: the int32 group sums [col][row][k / 32]
   // GLU write-back (slab with interleaved gate / up rows): the GLU of every (gate, up) pair,
   // requantized to Q8_1-MMQ blocks [nrows / 2 / 128][ncols], instead of the F32 output.
   std::uint8_t* glu_out;
@@ -316,53 +341,58 @@ struct Params {
   float limit;
 };
 
-template <bool kSlab>
+// K-major operand without swizzle: 8-row core matrices `sbo` bytes apart, the second half of the
+// K 16 in the tile at `zeros`.
+__device__ __forceinline__ std::uint64_t ScaleDesc(const unsigned char* tile,
+                                                   const unsigned char* zeros) {
+  const std::uint32_t lbo = (tc::Smem(zeros) - tc::Smem(tile)) >> 4;
+  return tc::SmemDesc(tile, false, 128) | (static_cast<std::uint64_t>(lbo & 0x3fffu) << 16);
+}
+
+// Both loads of a 16-row piece: the registers of the integers and of the scales are usable only
+// after this.
+__device__ __forceinline__ void PieceWait(std::uint32_t (&c)[16], std::uint32_t (&s)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(c[4]), "+r"(c[5]), "+r"(c[6]),
+                 "+r"(c[7]), "+r"(c[8]), "+r"(c[9]), "+r"(c[10]), "+r"(c[11]), "+r"(c[12]),
+                 "+r"(c[13]), "+r"(c[14]), "+r"(c[15]), "+r"(s[0]), "+r"(s[1]), "+r"(s[2]),
+                 "+r"(s[3]), "+r"(s[4]), "+r"(s[5]), "+r"(s[6]), "+r"(s[7]), "+r"(s[8]), "+r"(s[9]),
+                 "+r"(s[10]), "+r"(s[11]), "+r"(s[12]), "+r"(s[13]), "+r"(s[14]), "+r"(s[15])
+               :
+               : "memory");
+}
+
+template <bool kSlab, bool kSums>
 __global__ void __launch_bounds__(kThreads, 1)
 MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ CUtensorMap map_w,
              const __grid_constant__ CUtensorMap map_h, const __grid_constant__ CUtensorMap map_mw,
-             const Params p) {
+             const __grid_constant__ Params p) {
   const Desc& a = p.a;
-  extern __shared__ unsigned char raw_smem[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<std::uintptr_t>(raw_smem) + 1023) & ~static_cast<std::uintptr_t>(1023));
+  constexpr int kMins = kMinTiles<kSlab>;
+  extern __shared__ __align__(1024) unsigned char smem[];  // the swizzle's period
   unsigned char* w_tiles = smem;
   unsigned char* y_tiles = w_tiles + (kStages * kWBytes);
-  unsigned char* min_w = y_tiles + (kStages * kYBytes);  // [2] tiles: (-dmin * m) per weight row
-  unsigned char* min_y = min_w + (2 * kMinTileBytes);    // [2] tiles: s8 per token
-  unsigned char* raw = min_y + (2 * kMinTileBytes);      // [kRawStages] raw stages
-  float* scales = reinterpret_cast<float*>(raw + (kRawStages * kRawBytes));
-  Shared* sh = reinterpret_cast<Shared*>(reinterpret_cast<unsigned char*>(scales) +
-                                         (kStages * 2 * kScaleBytes));
-  // scales of stage s: ax[4][128] (weight rows, d * sc), bx[4][128] (tokens, d8)
-  auto stage_scales = [&](int s) { return scales + (static_cast<std::size_t>(s) * 2 * 512); };
+  unsigned char* min_w = y_tiles + (kStages * kYBytes);    // [kMins] tiles: (-dmin * m) per weight row
+  unsigned char* min_y = min_w + (kMins * kMinTileBytes);  // [kMins] tiles: s8 per token
+  unsigned char* scale_w = min_y + (kMins * kMinTileBytes);            // [kStages][group] d * sc
+  unsigned char* scale_y = scale_w + (kStages * kStageScaleBytes);     // [kStages][group] d8
+  unsigned char* zeros = scale_y + (kStages * kStageScaleBytes);
+  unsigned char* raw = zeros + kScaleTileBytes;                        // [kRawStages] raw stages
+  Shared* sh = reinterpret_cast<Shared*>(raw + (kRawStages * kRawBytes<kSlab>));
 
   const int warp = static_cast<int>(threadIdx.x) >> 5;
   const int lane = static_cast<int>(threadIdx.x) & 31;
   const int ksteps = a.k / kBK;
-
-  // The tile: weight rows [row0, row0 + 128) of expert e against sorted
-  // columns [col0, col0 + 128) of that expert's range [c_begin, c_end).
-  // With a worklist (built on the device from the expert bounds) grid row y
-  // names entry y: {expert, first column}; entry 0 holds the entry count.
-  int expert = static_cast<int>(blockIdx.z);
-  int col0;
-  if (p.worklist != nullptr) {
-    if (static_cast<int>(blockIdx.y) >= p.worklist[0]) return;
-    expert = p.worklist[1 + (2 * blockIdx.y)];
-    col0 = p.worklist[2 + (2 * blockIdx.y)];
-  } else {
-    const int c_begin = a.expert_bounds != nullptr ? a.expert_bounds[expert] : 0;
-    col0 = c_begin + (static_cast<int>(blockIdx.y) * kTileCols);
+  if ((tc::Smem(smem) & 1023u) != 0) {  // uniform: the tiles' layout needs it
+    if (threadIdx.x == 0) atomicAdd(p.faults, 1u);
+    return;
   }
-  const int c_end = a.expert_bounds != nullptr ? a.expert_bounds[expert + 1] : a.ncols;
-  const int row0 = static_cast<int>(blockIdx.x) * kTileRows;
-  if (col0 >= c_end) return;  // uniform for the CTA, before any barrier
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       tc::MbarInit(&sh->y_full[s], 1);
       tc::MbarInit(&sh->w_full[s], kDecodeWarps);
-      tc::MbarInit(&sh->empty[s], kEpilogueWarps);
+      tc::MbarInit(&sh->empty[s], 1);
     }
     for (int b = 0; b < kBuffers; ++b) {
       tc::MbarInit(&sh->tmem_full[b], 1);
@@ -376,9 +406,12 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
       tc::MbarInit(&sh->minw_full[t], 1);
       tc::MbarInit(&sh->min_free[t], 1);
     }
-    tc::MbarInit(&sh->min_full, 1);
     sh->abort = 0;
     tc::MbarInitFence();
+  }
+  if (threadIdx.x < kScaleTileBytes / 16) {
+    reinterpret_cast<uint4*>(zeros)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
+    tc::FenceProxyAsync();
   }
   if (warp == kMmaWarp) {
     tc::TmemAlloc(&sh->tmem_base, 512);
@@ -387,6 +420,38 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
   tc::TcFenceBefore();
   __syncthreads();
   tc::TcFenceAfter();
+  // All of the above runs beside the tail of the kernel before (the quantizer, the route, the
+  // relayout: everything below may be theirs).
+  GridLaunchDependents();
+  GridDependencyWait();
+
+  // A CTA takes tiles blockIdx.x, + gridDim.x, ...: weight rows [row0, row0 + 128) of an expert
+  // against sorted columns [col0, col0 + 128) of that expert's range, row tiles fastest.  With a
+  // worklist (built on the device from the expert bounds) column tile y names entry y: {expert,
+  // first column}; entry 0 holds the entry count.
+  const int row_tiles = (a.nrows + kTileRows - 1) / kTileRows;
+  const int col_tiles = p.worklist != nullptr ? min(p.worklist[0], p.col_tiles) : p.col_tiles;
+  const std::int64_t tiles = static_cast<std::int64_t>(row_tiles) * col_tiles *
+                             (p.worklist == nullptr && a.expert_bounds != nullptr ? a.experts : 1);
+  struct Tile {
+    int expert, row_tile, col0, c_end;
+  };
+  const auto tile_at = [&](std::int64_t i) {
+    Tile tile;
+    tile.row_tile = static_cast<int>(i % row_tiles);
+    const std::int64_t rest = i / row_tiles;
+    if (p.worklist != nullptr) {
+      tile.expert = p.worklist[1 + (2 * rest)];
+      tile.col0 = p.worklist[2 + (2 * rest)];
+    } else {
+      tile.expert = static_cast<int>(rest / col_tiles);
+      tile.col0 = (a.expert_bounds != nullptr ? a.expert_bounds[tile.expert] : 0) +
+                  (static_cast<int>(rest % col_tiles) * kTileCols);
+    }
+    tile.c_end = a.expert_bounds != nullptr ? a.expert_bounds[tile.expert + 1] : a.ncols;
+    return tile;  // nothing to do, for every role alike, when col0 >= c_end
+  };
+
   const std::uint32_t tmem = sh->tmem_base;
   volatile std::uint32_t* abort_flag = &sh->abort;
   auto give_up = [&]() {
@@ -401,399 +466,473 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
       tc::PrefetchMap(&map_w);
       tc::PrefetchMap(&map_h);
       if constexpr (kSlab) tc::PrefetchMap(&map_mw);
-      for (int ks = 0; ks < ksteps && !*abort_flag; ++ks) {
-        if ((ks & 1) == 0) {
-          // One super-block column (k-steps ks, ks + 1): the tokens' block headers
-          // and, raw, the weight rows' blocks, for the decode warps.
-          const int column = ks >> 1;
-          const int rs = column % kRawStages;
-          if (!tc::MbarWaitSleep(&sh->raw_empty[rs], ((column / kRawStages) & 1) ^ 1, 128)) {
-            give_up();
-            break;
-          }
-          unsigned char* stage = raw + (rs * kRawBytes);
-          tc::MbarExpectTx(&sh->raw_full[rs], kSlab ? 2 * kRawHBytes : kRawBytes);
-          if constexpr (!kSlab) {
-            asm volatile(
-                "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                " [%0], [%1, {%3, %4, %5}], [%2];"
-                ::"r"(tc::Smem(stage)), "l"(&map_w), "r"(tc::Smem(&sh->raw_full[rs])),
-                  "r"(column * 144), "r"(row0), "r"(expert)
-                : "memory");
-          }
-          asm volatile(
-              "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-              " [%0], [%1, {%3, %4, %5}], [%2];"
-              ::"r"(tc::Smem(stage + kRawWBytes)), "l"(&map_h), "r"(tc::Smem(&sh->raw_full[rs])),
-                "r"(0), "r"(col0), "r"(ks)
-              : "memory");
-        }
-        if constexpr (kSlab) {
-          // Every 16 k-steps a tile of the weight rows' min operands.
-          if (ks % kMinSteps == 0) {
-            const int mt = (ks / kMinSteps) & 1;
-            if (ks >= 2 * kMinSteps &&
-                !tc::MbarWaitSleep(&sh->min_free[mt], ((ks / (2 * kMinSteps)) - 1) & 1, 128)) {
+      std::uint32_t it = 0, column = 0, mins = 0;  // k-steps, super-block columns, min tiles so far
+      bool ok = true;
+      for (std::int64_t i = blockIdx.x; i < tiles && ok && !*abort_flag; i += gridDim.x) {
+        const Tile tile = tile_at(i);
+        if (tile.col0 >= tile.c_end) continue;
+        const int expert = tile.expert, col0 = tile.col0, row0 = tile.row_tile * kTileRows;
+        for (int ks = 0; ks < ksteps; ++ks, ++it) {
+          if ((ks & 1) == 0) {
+            // One super-block column (k-steps ks, ks + 1): the tokens' block headers and the
+            // weight rows' scales (or, raw, their blocks), for the decode warps.
+            const int rs = static_cast<int>(column % kRawStages);
+            ok = tc::MbarWaitSleep(&sh->raw_empty[rs], ((column / kRawStages) & 1) ^ 1, 128);
+            if (!ok) {
               give_up();
               break;
             }
-            tc::MbarExpectTx(&sh->minw_full[mt], kMinTileBytes);
+            unsigned char* stage = raw + (rs * kRawBytes<kSlab>);
+            tc::MbarExpectTx(&sh->raw_full[rs], kRawBytes<kSlab>);
+            if constexpr (kSlab) {
+              // k is a multiple of 256: the two k-steps' tiles are 4 KB in a row
+              const float* src = p.ax + ((((static_cast<std::int64_t>(expert) * p.ax_row_tiles) +
+                                           tile.row_tile) * p.ax_ksteps + ks) * 512);
+              tc::BulkLoad(stage, src, 2 * kAxBytes, &sh->raw_full[rs]);
+            } else {
+              asm volatile(
+                  "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                  " [%0], [%1, {%3, %4, %5}], [%2];"
+                  ::"r"(tc::Smem(stage)), "l"(&map_w), "r"(tc::Smem(&sh->raw_full[rs])),
+                    "r"((ks >> 1) * 144), "r"(row0), "r"(expert)
+                  : "memory");
+            }
             asm volatile(
                 "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
                 " [%0], [%1, {%3, %4, %5}], [%2];"
-                ::"r"(tc::Smem(min_w + (mt * kMinTileBytes))), "l"(&map_mw),
-                  "r"(tc::Smem(&sh->minw_full[mt])), "r"((ks / kMinSteps) * 128), "r"(row0),
-                  "r"(expert)
+                ::"r"(tc::Smem(stage + kRawWBytes<kSlab>)), "l"(&map_h),
+                  "r"(tc::Smem(&sh->raw_full[rs])), "r"(0), "r"(col0), "r"(ks)
                 : "memory");
+            ++column;
           }
-        }
-        const int s = ks % kStages;
-        if (!tc::MbarWaitSleep(&sh->empty[s], ((ks / kStages) & 1) ^ 1, 256)) {
-          give_up();
-          break;
-        }
-        tc::MbarExpectTx(&sh->y_full[s], kSlab ? kYBytes + kWBytes + kScaleBytes : kYBytes);
-        asm volatile(
-            "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-            " [%0], [%1, {%3, %4, %5}], [%2];"
-            ::"r"(tc::Smem(y_tiles + (s * kYBytes))), "l"(&map_y), "r"(tc::Smem(&sh->y_full[s])),
-              "r"(0), "r"(col0), "r"(ks)
-            : "memory");
-        if constexpr (kSlab) {
+          if constexpr (kSlab) {
+            // Every 16 k-steps a tile of the weight rows' min operands.
+            if (ks % kMinSteps == 0) {
+              const int mt = static_cast<int>(mins % kMins);
+              if (mins >= kMins) ok = tc::MbarWaitSleep(&sh->min_free[mt], ((mins / kMins) - 1) & 1, 128);
+              if (!ok) {
+                give_up();
+                break;
+              }
+              ++mins;
+              tc::MbarExpectTx(&sh->minw_full[mt], kMinTileBytes);
+              asm volatile(
+                  "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                  " [%0], [%1, {%3, %4, %5}], [%2];"
+                  ::"r"(tc::Smem(min_w + (mt * kMinTileBytes))), "l"(&map_mw),
+                    "r"(tc::Smem(&sh->minw_full[mt])), "r"((ks / kMinSteps) * 128), "r"(row0),
+                    "r"(expert)
+                  : "memory");
+            }
+          }
+          const int s = static_cast<int>(it % kStages);
+          ok = tc::MbarWaitSleep(&sh->empty[s], ((it / kStages) & 1) ^ 1, 64);
+          if (!ok) {
+            give_up();
+            break;
+          }
+          tc::MbarExpectTx(&sh->y_full[s], kSlab ? kYBytes + kWBytes : kYBytes);
           asm volatile(
               "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
               " [%0], [%1, {%3, %4, %5}], [%2];"
-              ::"r"(tc::Smem(w_tiles + (s * kWBytes))), "l"(&map_w), "r"(tc::Smem(&sh->y_full[s])),
-                "r"(ks * kBK), "r"(row0), "r"(expert)
+              ::"r"(tc::Smem(y_tiles + (s * kYBytes))), "l"(&map_y), "r"(tc::Smem(&sh->y_full[s])),
+                "r"(0), "r"(col0), "r"(ks)
               : "memory");
-          const float* src = p.ax + ((((static_cast<std::int64_t>(expert) * p.ax_row_tiles) +
-                                       blockIdx.x) * p.ax_ksteps + ks) * 512);
-          tc::BulkLoad(stage_scales(s), src, kScaleBytes, &sh->y_full[s]);
+          if constexpr (kSlab) {
+            asm volatile(
+                "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                " [%0], [%1, {%3, %4, %5}], [%2];"
+                ::"r"(tc::Smem(w_tiles + (s * kWBytes))), "l"(&map_w), "r"(tc::Smem(&sh->y_full[s])),
+                  "r"(ks * kBK), "r"(row0), "r"(expert)
+                : "memory");
+          }
         }
       }
     }
-  } else if (warp >= 1 && warp <= kDecodeWarps) {
+  } else if (warp >= kFirstDecodeWarp && warp < kFirstEpilogueWarp) {
     // ------------------------------------------------------------ decode
-    const int t0 = (static_cast<int>(threadIdx.x) - 32);  // first weight row / token of this thread
-    // Rows past the matrix and tokens past the batch arrive as zero blocks (TMA's
-    // fill): zero scales, zero codes, nothing stored for them.
-    for (int ks = 0; ks < ksteps && !*abort_flag; ++ks) {
-      const int s = ks % kStages;
-      const int half = ks & 1;
-      const int column = ks >> 1;
-      const int rs = column % kRawStages;
-      const int mt = (ks / kMinSteps) & 1;  // the tile of min operands this k-step writes into
-      bool ok = true;
-      if (lane == 0) {
-        if (half == 0) ok = tc::MbarWait(&sh->raw_full[rs], (column / kRawStages) & 1);
-        ok = ok && tc::MbarWaitSleep(&sh->empty[s], ((ks / kStages) & 1) ^ 1, 64);
-        // ... and the tensor core is done with the min tile's contents of 32 k-steps ago
-        if (ks >= 2 * kMinSteps && ks % kMinSteps == 0) {
-          ok = ok && tc::MbarWait(&sh->min_free[mt], ((ks / (2 * kMinSteps)) - 1) & 1);
+    // A thread prepares weight rows and tokens t0 and t0 + 64 of every k-step.  Rows past the
+    // matrix and tokens past the batch arrive as zero blocks (TMA's fill): zero scales, zero
+    // codes, nothing stored for them.
+    const int t0 = static_cast<int>(threadIdx.x) - (kFirstDecodeWarp * 32);
+    std::uint32_t it = 0, column = 0, mins = 0;
+    bool ok = true;
+    for (std::int64_t i = blockIdx.x; i < tiles && ok && !*abort_flag; i += gridDim.x) {
+      const Tile tile = tile_at(i);
+      if (tile.col0 >= tile.c_end) continue;
+      for (int ks = 0; ks < ksteps; ++ks, ++it) {
+        const int s = static_cast<int>(it % kStages);
+        const int half = ks & 1;
+        const int rs = static_cast<int>(column % kRawStages);
+        const int mt = static_cast<int>(mins % kMins);  // the tile of min operands this k-step writes into
+        if (lane == 0) {
+          if (half == 0) ok = tc::MbarWait(&sh->raw_full[rs], (column / kRawStages) & 1);
+          ok = ok && tc::MbarWait(&sh->empty[s], ((it / kStages) & 1) ^ 1);
+          // ... and the tensor core is done with the min tile's contents of kMins tiles ago
+          if (mins >= kMins && ks % kMinSteps == 0) {
+            ok = ok && tc::MbarWait(&sh->min_free[mt], ((mins / kMins) - 1) & 1);
+          }
         }
-      }
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      if (!ok) {
-        if (lane == 0) give_up();
-        break;
-      }
-      const unsigned char* stage = raw + (rs * kRawBytes);
-      float* sc = stage_scales(s);
-      const int kk = ks % kMinSteps;
+        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+        if (!ok) {
+          if (lane == 0) give_up();
+          break;
+        }
+        const unsigned char* stage = raw + (rs * kRawBytes<kSlab>);
+        const int kk = ks % kMinSteps;
 #pragma unroll  // the rows of a thread are independent: their latencies overlap
-      for (int t = t0; t < kTileRows; t += kDecodeWarps * 32) {
-        // Row t of a min tile, the four halves of this k-step: byte (ks % 16) * 8 of
-        // the 128-byte row, 16-byte chunks swizzled like the int8 tiles.
-        const int at = ((t >> 3) * 1024) + ((t & 7) * 128) + ((((kk >> 1) ^ (t & 7))) * 16) +
-                       ((kk & 1) * 8);
-        if constexpr (!kSlab) {
-          const unsigned char* sb = stage + (t * 144);
-          const uint4 head = *reinterpret_cast<const uint4*>(sb);
-          uint4 q[4];
+        for (int t = t0; t < kTileRows; t += kDecodeWarps * 32) {
+          const int row_at = ((t >> 3) * 128) + ((t & 7) * 16);  // row t of a scale tile
+          unsigned char* sw = scale_w + (s * kStageScaleBytes) + row_at;
+          unsigned char* sy = scale_y + (s * kStageScaleBytes) + row_at;
+          // Row t of a min tile, the four halves of this k-step: byte (ks % 16) * 8 of
+          // the 128-byte row, 16-byte chunks swizzled like the int8 tiles.
+          const int at = ((t >> 3) * 1024) + ((t & 7) * 128) + ((((kk >> 1) ^ (t & 7))) * 16) +
+                         ((kk & 1) * 8);
+          if constexpr (kSlab) {
+            // (d * sc)_half comes widened to F32: back to half precision, exactly.
+            const float* ax = reinterpret_cast<const float*>(stage + (half * kAxBytes)) + t;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            q[i] = *reinterpret_cast<const uint4*>(sb + 16 + (half * 64) + (i * 16));
-          }
-          // int8 codes into the swizzled K-major tile: row t, 16-byte chunk j at j ^ (t % 8)
-          unsigned char* wt = w_tiles + (s * kWBytes) + ((t >> 3) * 1024) + ((t & 7) * 128);
+            for (int gl = 0; gl < 4; ++gl) {
+              *reinterpret_cast<uint4*>(sw + (gl * kScaleTileBytes)) =
+                  make_uint4(__half_as_ushort(__float2half_rn(ax[gl * 128])), 0u, 0u, 0u);
+            }
+          } else {
+            const unsigned char* sb = stage + (t * 144);
+            const uint4 head = *reinterpret_cast<const uint4*>(sb);
+            uint4 q[4];
 #pragma unroll
-          for (int cc = 0; cc < 2; ++cc) {
-            const uint4 lo0 = make_uint4(q[2 * cc].x & 0x0f0f0f0fu, q[2 * cc].y & 0x0f0f0f0fu,
-                                         q[2 * cc].z & 0x0f0f0f0fu, q[2 * cc].w & 0x0f0f0f0fu);
-            const uint4 lo1 = make_uint4(q[2 * cc + 1].x & 0x0f0f0f0fu, q[2 * cc + 1].y & 0x0f0f0f0fu,
-                                         q[2 * cc + 1].z & 0x0f0f0f0fu, q[2 * cc + 1].w & 0x0f0f0f0fu);
-            const uint4 hi0 = make_uint4((q[2 * cc].x >> 4) & 0x0f0f0f0fu, (q[2 * cc].y >> 4) & 0x0f0f0f0fu,
-                                         (q[2 * cc].z >> 4) & 0x0f0f0f0fu, (q[2 * cc].w >> 4) & 0x0f0f0f0fu);
-            const uint4 hi1 = make_uint4((q[2 * cc + 1].x >> 4) & 0x0f0f0f0fu, (q[2 * cc + 1].y >> 4) & 0x0f0f0f0fu,
-                                         (q[2 * cc + 1].z >> 4) & 0x0f0f0f0fu, (q[2 * cc + 1].w >> 4) & 0x0f0f0f0fu);
-            const int j = cc * 4;  // groups 2cc (chunks j, j+1) and 2cc+1 (chunks j+2, j+3)
-            *reinterpret_cast<uint4*>(wt + (((j + 0) ^ (t & 7)) * 16)) = lo0;
-            *reinterpret_cast<uint4*>(wt + (((j + 1) ^ (t & 7)) * 16)) = lo1;
-            *reinterpret_cast<uint4*>(wt + (((j + 2) ^ (t & 7)) * 16)) = hi0;
-            *reinterpret_cast<uint4*>(wt + (((j + 3) ^ (t & 7)) * 16)) = hi1;
+            for (int i = 0; i < 4; ++i) {
+              q[i] = *reinterpret_cast<const uint4*>(sb + 16 + (half * 64) + (i * 16));
+            }
+            // int8 codes into the swizzled K-major tile: row t, 16-byte chunk j at j ^ (t % 8)
+            unsigned char* wt = w_tiles + (s * kWBytes) + ((t >> 3) * 1024) + ((t & 7) * 128);
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc) {
+              const uint4 lo0 = make_uint4(q[2 * cc].x & 0x0f0f0f0fu, q[2 * cc].y & 0x0f0f0f0fu,
+                                           q[2 * cc].z & 0x0f0f0f0fu, q[2 * cc].w & 0x0f0f0f0fu);
+              const uint4 lo1 = make_uint4(q[2 * cc + 1].x & 0x0f0f0f0fu, q[2 * cc + 1].y & 0x0f0f0f0fu,
+                                           q[2 * cc + 1].z & 0x0f0f0f0fu, q[2 * cc + 1].w & 0x0f0f0f0fu);
+              const uint4 hi0 = make_uint4((q[2 * cc].x >> 4) & 0x0f0f0f0fu, (q[2 * cc].y >> 4) & 0x0f0f0f0fu,
+                                           (q[2 * cc].z >> 4) & 0x0f0f0f0fu, (q[2 * cc].w >> 4) & 0x0f0f0f0fu);
+              const uint4 hi1 = make_uint4((q[2 * cc + 1].x >> 4) & 0x0f0f0f0fu, (q[2 * cc + 1].y >> 4) & 0x0f0f0f0fu,
+                                           (q[2 * cc + 1].z >> 4) & 0x0f0f0f0fu, (q[2 * cc + 1].w >> 4) & 0x0f0f0f0fu);
+              const int j = cc * 4;  // groups 2cc (chunks j, j+1) and 2cc+1 (chunks j+2, j+3)
+              *reinterpret_cast<uint4*>(wt + (((j + 0) ^ (t & 7)) * 16)) = lo0;
+              *reinterpret_cast<uint4*>(wt + (((j + 1) ^ (t & 7)) * 16)) = lo1;
+              *reinterpret_cast<uint4*>(wt + (((j + 2) ^ (t & 7)) * 16)) = hi0;
+              *reinterpret_cast<uint4*>(wt + (((j + 3) ^ (t & 7)) * 16)) = hi1;
+            }
+            // The four groups' half products (d * sc, -dmin * m): GGML's tile loader
+            // multiplies in half precision.
+            const __half d = __ushort_as_half(static_cast<unsigned short>(head.x & 0xffffu));
+            const __half dmin = __hneg(__ushort_as_half(static_cast<unsigned short>(head.x >> 16)));
+            std::uint32_t mins[4];
+#pragma unroll
+            for (int gl = 0; gl < 4; ++gl) {
+              int scv, mnv;
+              ScaleAndMin(head.y, head.z, head.w, (half * 4) + gl, &scv, &mnv);
+              *reinterpret_cast<uint4*>(sw + (gl * kScaleTileBytes)) =
+                  make_uint4(__half_as_ushort(__hmul(d, __int2half_rn(scv))), 0u, 0u, 0u);
+              mins[gl] = __half_as_ushort(__hmul(dmin, __int2half_rn(mnv)));
+            }
+            *reinterpret_cast<uint2*>(min_w + (mt * kMinTileBytes) + at) =
+                make_uint2(mins[0] | (mins[1] << 16), mins[2] | (mins[3] << 16));
           }
-          // The four groups' half products (d * sc, -dmin * m): GGML's tile loader
-          // multiplies in half precision.
-          const __half d = __ushort_as_half(static_cast<unsigned short>(head.x & 0xffffu));
-          const __half dmin = __hneg(__ushort_as_half(static_cast<unsigned short>(head.x >> 16)));
-          std::uint32_t mins[4];
+          // The token's header of this k-step: four (d8, s8) pairs.
+          const uint4 ds = *reinterpret_cast<const uint4*>(stage + kRawWBytes<kSlab> +
+                                                           (half * kRawHBytes) + (t * 16));
+          const std::uint32_t dsw[4] = {ds.x, ds.y, ds.z, ds.w};
 #pragma unroll
           for (int gl = 0; gl < 4; ++gl) {
-            int scv, mnv;
-            ScaleAndMin(head.y, head.z, head.w, (half * 4) + gl, &scv, &mnv);
-            sc[(gl * 128) + t] = __half2float(__hmul(d, __int2half_rn(scv)));
-            mins[gl] = __half_as_ushort(__hmul(dmin, __int2half_rn(mnv)));
+            *reinterpret_cast<uint4*>(sy + (gl * kScaleTileBytes)) = make_uint4(dsw[gl] & 0xffffu, 0u, 0u, 0u);
           }
-          *reinterpret_cast<uint2*>(min_w + (mt * kMinTileBytes) + at) =
-              make_uint2(mins[0] | (mins[1] << 16), mins[2] | (mins[3] << 16));
-        }
-        // The token's header of this k-step: four (d8, s8) pairs.
-        const uint4 ds =
-            *reinterpret_cast<const uint4*>(stage + kRawWBytes + (half * kRawHBytes) + (t * 16));
-        const std::uint32_t dsw[4] = {ds.x, ds.y, ds.z, ds.w};
-#pragma unroll
-        for (int gl = 0; gl < 4; ++gl) sc[512 + (gl * 128) + t] = HalfBitsToFloat(dsw[gl] & 0xffffu);
-        *reinterpret_cast<uint2*>(min_y + (mt * kMinTileBytes) + at) =
-            make_uint2((dsw[0] >> 16) | (dsw[1] & 0xffff0000u), (dsw[2] >> 16) | (dsw[3] & 0xffff0000u));
-        // The last FP16 MMA reads 16 groups: zero what the k range leaves unwritten.
-        if (ks == ksteps - 1) {
-          for (int pad = ks + 1; pad % 4 != 0; ++pad) {
-            const int pk = pad % kMinSteps;
-            const int pat = ((t >> 3) * 1024) + ((t & 7) * 128) + ((((pk >> 1) ^ (t & 7))) * 16) +
-                            ((pk & 1) * 8);
-            if constexpr (!kSlab) {
-              *reinterpret_cast<uint2*>(min_w + (mt * kMinTileBytes) + pat) = make_uint2(0u, 0u);
+          *reinterpret_cast<uint2*>(min_y + (mt * kMinTileBytes) + at) =
+              make_uint2((dsw[0] >> 16) | (dsw[1] & 0xffff0000u), (dsw[2] >> 16) | (dsw[3] & 0xffff0000u));
+          // The last FP16 MMA of the min terms reads 16 groups: zero what the k range leaves unwritten.
+          if (ks == ksteps - 1) {
+            for (int pad = ks + 1; pad % 4 != 0; ++pad) {
+              const int pk = pad % kMinSteps;
+              const int pat = ((t >> 3) * 1024) + ((t & 7) * 128) + ((((pk >> 1) ^ (t & 7))) * 16) +
+                              ((pk & 1) * 8);
+              if constexpr (!kSlab) {
+                *reinterpret_cast<uint2*>(min_w + (mt * kMinTileBytes) + pat) = make_uint2(0u, 0u);
+              }
+              *reinterpret_cast<uint2*>(min_y + (mt * kMinTileBytes) + pat) = make_uint2(0u, 0u);
             }
-            *reinterpret_cast<uint2*>(min_y + (mt * kMinTileBytes) + pat) = make_uint2(0u, 0u);
           }
         }
-      }
-      tc::FenceProxyAsync();  // generic-proxy writes, read by the tensor core's proxy
-      __syncwarp();
-      if (lane == 0) {
-        if (half == 1 || ks == ksteps - 1) tc::MbarArrive(&sh->raw_empty[rs]);  // the raw stage is read
-        tc::MbarArrive(&sh->w_full[s]);
+        tc::FenceProxyAsync();  // generic-proxy writes, read by the tensor core's proxy
+        __syncwarp();
+        if (lane == 0) {
+          if (half == 1) tc::MbarArrive(&sh->raw_empty[rs]);  // the raw stage is read
+          tc::MbarArrive(&sh->w_full[s]);
+        }
+        if (half == 1) ++column;
+        if (ks % kMinSteps == kMinSteps - 1 || ks == ksteps - 1) ++mins;
       }
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      // A (M, the TMEM lanes): tokens, signed int8.  B (N, the TMEM columns): weight
-      // rows, unsigned codes.
-      const std::uint32_t idesc = tc::IdescI8(kTileCols, kTileRows, true, false);
-      std::uint32_t group = 0;
-      for (int ks = 0; ks < ksteps && !*abort_flag; ++ks) {
-        const int s = ks % kStages;
-        if (!tc::MbarWait(&sh->w_full[s], (ks / kStages) & 1) ||
-            !tc::MbarWait(&sh->y_full[s], (ks / kStages) & 1)) {
-          give_up();
+    // The whole warp walks the loop and one elected lane issues: from inside a one-lane branch
+    // every MMA and commit held the thread 60-70 cycles.
+    const bool elected = tc::ElectOne();
+    // A (M, the TMEM lanes): tokens, signed int8.  B (N, the TMEM columns): weight
+    // rows, unsigned codes.
+    const std::uint32_t idesc = tc::IdescI8(kTileCols, kTileRows, true, false);
+    const std::uint32_t fdesc = tc::IdescF16(kTileCols, kTileRows);
+    std::uint32_t turn = 0, it = 0, mins = 0;  // turn: of the TMEM buffers
+    bool ok = true;
+    for (std::int64_t i = blockIdx.x; i < tiles && ok && !*abort_flag; i += gridDim.x) {
+      const Tile tile = tile_at(i);
+      if (tile.col0 >= tile.c_end) continue;
+      for (int ks = 0; ks < ksteps; ++ks, ++it) {
+        const int s = static_cast<int>(it % kStages);
+        ok = tc::MbarWait(&sh->w_full[s], (it / kStages) & 1) &&
+             tc::MbarWait(&sh->y_full[s], (it / kStages) & 1);
+        if (!__all_sync(0xffffffffu, ok)) {
+          ok = false;
           break;
         }
         tc::TcFenceAfter();
         const std::uint64_t wdesc = tc::SmemDesc(w_tiles + (s * kWBytes), true, 1024);
         const std::uint64_t ydesc = tc::SmemDesc(y_tiles + (s * kYBytes), true, 1024);
-        for (int gl = 0; gl < 4; ++gl, ++group) {
-          const int b = static_cast<int>(group % kBuffers);
-          if (!tc::MbarWait(&sh->tmem_empty[b], ((group / kBuffers) & 1u) ^ 1u)) {
-            give_up();
+        const unsigned char* sw = scale_w + (s * kStageScaleBytes);
+        const unsigned char* sy = scale_y + (s * kStageScaleBytes);
+#pragma unroll
+        for (int gl = 0; gl < 4; ++gl, ++turn) {
+          const int b = static_cast<int>(turn % kBuffers);
+          const std::uint64_t swd = ScaleDesc(sw + (gl * kScaleTileBytes), zeros);
+          const std::uint64_t syd = ScaleDesc(sy + (gl * kScaleTileBytes), zeros);
+          ok = tc::MbarWait(&sh->tmem_empty[b], ((turn / kBuffers) & 1u) ^ 1u);
+          if (!__all_sync(0xffffffffu, ok)) {
+            ok = false;
             break;
           }
           tc::TcFenceAfter();
-          tc::MmaI8(tmem + (b * kTileRows), ydesc + (gl * 2), wdesc + (gl * 2), idesc, false);
-          tc::TcCommit(&sh->tmem_full[b]);
-        }
-        // Every fourth k-step completes 16 groups of min operands: one FP16 MMA
-        // (K 16) adds their products to the F32 sum.
-        if (ks % 4 == 3 || ks == ksteps - 1) {
-          const int mt = (ks / kMinSteps) & 1;
-          const int q = (ks % kMinSteps) / 4;  // 32 bytes along the swizzled row each
-          if constexpr (kSlab) {
-            if (q == 0 && !tc::MbarWait(&sh->minw_full[mt], (ks / (2 * kMinSteps)) & 1)) {
-              give_up();
-              break;
-            }
-            tc::TcFenceAfter();
+          if (elected) {
+            const std::uint32_t d = tmem + (b * kBufferColumns);
+            tc::MmaI8(d, ydesc + (gl * 2), wdesc + (gl * 2), idesc, false);
+            tc::MmaF16(d + kScaleColumn, syd, swd, fdesc, false);
+            tc::TcCommit(&sh->tmem_full[b]);
+            if (gl == 3) tc::TcCommit(&sh->empty[s]);
           }
-          tc::MmaF16(tmem + kMinColumn, tc::SmemDesc(min_y + (mt * kMinTileBytes), true, 1024) + (q * 2),
-                     tc::SmemDesc(min_w + (mt * kMinTileBytes), true, 1024) + (q * 2),
-                     tc::IdescF16(kTileCols, kTileRows), ks >= 4);
-          if (ks % kMinSteps == kMinSteps - 1) tc::TcCommit(&sh->min_free[mt]);
-          if (ks == ksteps - 1) tc::TcCommit(&sh->min_full);
         }
+        if (!ok) break;
+        // Every 16 k-steps, and at the end, the min terms of the tile: up to four FP16 MMAs (K 16
+        // each, the operands of four k-steps) into the next buffer.
+        if (ks % kMinSteps == kMinSteps - 1 || ks == ksteps - 1) {
+          const int mt = static_cast<int>(mins % kMins);
+          const int b = static_cast<int>(turn % kBuffers);
+          ok = tc::MbarWait(&sh->tmem_empty[b], ((turn / kBuffers) & 1u) ^ 1u);
+          if constexpr (kSlab) ok = ok && tc::MbarWait(&sh->minw_full[mt], (mins / kMins) & 1);
+          if (!__all_sync(0xffffffffu, ok)) {
+            ok = false;
+            break;
+          }
+          tc::TcFenceAfter();
+          if (elected) {
+            const std::uint64_t myd = tc::SmemDesc(min_y + (mt * kMinTileBytes), true, 1024);
+            const std::uint64_t mwd = tc::SmemDesc(min_w + (mt * kMinTileBytes), true, 1024);
+            const int last = (ks % kMinSteps) / 4;
+            for (int q = 0; q <= last; ++q) {  // 32 bytes along the swizzled row each
+              tc::MmaF16(tmem + (b * kBufferColumns), myd + (q * 2), mwd + (q * 2), fdesc, q > 0);
+            }
+            tc::TcCommit(&sh->tmem_full[b]);
+            tc::TcCommit(&sh->min_free[mt]);
+          }
+          ++turn;
+          ++mins;
+        }
+        __syncwarp();
       }
     }
+    if (!ok && elected) give_up();
   } else {
     // ------------------------------------------------------------ epilogue
+    // acc += C * (d8 * d sc) for 64 rows a thread, 16 at a time: a piece is two TMEM loads, the
+    // integers and the scale products the tensor core formed beside them, one conversion a value
+    // and one packed multiply-add a pair.
     const int ew = warp - kFirstEpilogueWarp;
     const int quadrant = warp & 3;          // TMEM lanes this warp may touch
     const int rowgroup = ew >> 2;           // which kEpilogueRows weight rows
     const int tt = (quadrant * 32) + lane;  // token of the tile
-    const std::uint32_t lane_base = static_cast<std::uint32_t>(quadrant * 32) << 16;
+    const std::uint32_t base =
+        tmem + (static_cast<std::uint32_t>(quadrant * 32) << 16) + (rowgroup * kEpilogueRows);
     std::uint64_t acc2[kEpilogueRows / 2];  // rows 2i, 2i + 1
+    std::uint32_t ca[16], sa[16], cb[16], sb[16];  // two pieces
+    std::uint32_t turn = 0;
+    bool ok = true, ahead = false;  // ahead: the group's first piece is already on its way
+    const auto fold = [&](int piece, const std::uint32_t (&c)[16], const std::uint32_t (&s)[16]) {
 #pragma unroll
-    for (int i = 0; i < kEpilogueRows / 2; ++i) acc2[i] = 0ull;
-    const int col = col0 + tt;  // this thread's sorted column
-    bool ok = true;
-    int bb = 0;                  // the group's TMEM buffer and its use's parity
-    std::uint32_t parity = 0;
-    for (int ks = 0; ks < ksteps && ok && !*abort_flag; ++ks) {
-      const int s = ks % kStages;
-      const float* sc = stage_scales(s);
+      for (int i = 0; i < 8; ++i) {
+        acc2[(piece * 8) + i] =
+            Fma2(Pack2(__int2float_rn(static_cast<int>(c[2 * i])), __int2float_rn(static_cast<int>(c[(2 * i) + 1]))),
+                 Pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[(2 * i) + 1])),
+                 acc2[(piece * 8) + i]);
+      }
+    };
+    const auto check = [&](int group, int piece, int col, int row0, const std::uint32_t (&c)[16]) {
+      // verification: the exact group sums, before any float touches them
 #pragma unroll
-      for (int gl = 0; gl < 4; ++gl) {
-        if (!ok) break;
-        ok = tc::MbarWait(&sh->tmem_full[bb], parity);  // every lane polls: no shuffle after
-        if (!__all_sync(0xffffffffu, ok)) {
-          if (lane == 0) give_up();
-          ok = false;
-          break;
+      for (int j = 0; j < 16; ++j) {
+        const int row = row0 + (rowgroup * kEpilogueRows) + (piece * 16) + j;
+        if (row < a.nrows) {
+          p.sums[((static_cast<std::size_t>(col) * a.nrows + row) * (a.k / 32)) + group] =
+              static_cast<std::int32_t>(c[j]);
         }
-        tc::TcFenceAfter();
-        const std::uint32_t at = tmem + lane_base + (bb * kTileRows) + (rowgroup * kEpilogueRows);
-        // The thread's 32 rows at once, then the buffer goes straight back to the
-        // tensor core: the fold below overlaps the next groups' MMAs.
-        std::uint32_t r[32];
-        tc::TmemLoad32(at, r);
-        const float bx = sc[512 + (gl * 128) + tt];
-        const float4* ax4 = reinterpret_cast<const float4*>(sc + (gl * 128) + (rowgroup * kEpilogueRows));
-        tc::TmemLoadWait();
+      }
+    };
+    const auto load = [&](std::uint32_t from, std::uint32_t (&c)[16], std::uint32_t (&s)[16]) {
+      tc::TmemLoad16(from, c);
+      tc::TmemLoad16(from + kScaleColumn, s);
+    };
+    const int groups = ksteps * 4;
+    for (std::int64_t i = blockIdx.x; i < tiles && ok && !*abort_flag; i += gridDim.x) {
+      const Tile tile = tile_at(i);
+      const int c_end = tile.c_end;
+      if (tile.col0 >= c_end) continue;
+      const int row0 = tile.row_tile * kTileRows;
+      const int col = tile.col0 + tt;  // this thread's sorted column
+#pragma unroll
+      for (int j = 0; j < kEpilogueRows / 2; ++j) acc2[j] = 0ull;
+      for (int g = 0; g < groups; ++g) {
+        const int b = static_cast<int>(turn % kBuffers);
+        const std::uint32_t at = base + (b * kBufferColumns);
+        if (!ahead) {
+          ok = tc::MbarWait(&sh->tmem_full[b], (turn / kBuffers) & 1u);
+          if (!__all_sync(0xffffffffu, ok)) {
+            ok = false;
+            break;
+          }
+          tc::TcFenceAfter();
+          load(at, ca, sa);
+        }
+        ++turn;
+        PieceWait(ca, sa);
+        load(at + 16, cb, sb);
+        if constexpr (kSums) {
+          if (col < c_end) check(g, 0, col, row0, ca);
+        }
+        fold(0, ca, sa);
+        PieceWait(cb, sb);
+        load(at + 32, ca, sa);
+        if constexpr (kSums) {
+          if (col < c_end) check(g, 1, col, row0, cb);
+        }
+        fold(1, cb, sb);
+        PieceWait(ca, sa);
+        load(at + 48, cb, sb);
+        if constexpr (kSums) {
+          if (col < c_end) check(g, 2, col, row0, ca);
+        }
+        fold(2, ca, sa);
+        PieceWait(cb, sb);
+        // The buffer goes back to the tensor core; the next group's first piece, if it is there
+        // already, is requested under this one's last fold.
         tc::TcFenceBefore();
         __syncwarp();
-        if (lane == 0) tc::MbarArrive(&sh->tmem_empty[bb]);
-        if (p.sums != nullptr) {
-          // verification: the exact group sums, before any float touches them
-          if (col < c_end) {
-            const int groups = a.k / 32;
+        if (lane == 0) tc::MbarArrive(&sh->tmem_empty[b]);
+        const bool tail = (g & 63) == 63 || g == groups - 1;
+        ahead = false;
+        if (!tail) {
+          const int nb = static_cast<int>(turn % kBuffers);
+          ahead = __all_sync(0xffffffffu, tc::MbarTest(&sh->tmem_full[nb], (turn / kBuffers) & 1u));
+          if (ahead) {
+            tc::TcFenceAfter();
+            load(base + (nb * kBufferColumns), ca, sa);
+          }
+        }
+        if constexpr (kSums) {
+          if (col < c_end) check(g, 3, col, row0, cb);
+        }
+        fold(3, cb, sb);
+        if (tail) {
+          // The min terms of 64 groups: sum of (-dmin * m) * s8, taken by the tensor core.
+          const int mb = static_cast<int>(turn % kBuffers);
+          ok = tc::MbarWait(&sh->tmem_full[mb], (turn / kBuffers) & 1u);
+          if (!__all_sync(0xffffffffu, ok)) {
+            ok = false;
+            break;
+          }
+          tc::TcFenceAfter();
+          ++turn;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int row = row0 + (rowgroup * kEpilogueRows) + j;
-              if (row < a.nrows) {
-                p.sums[((static_cast<std::size_t>(col) * a.nrows + row) * groups) + (ks * 4) + gl] =
-                    static_cast<std::int32_t>(r[j]);
-              }
+          for (int piece = 0; piece < 4; ++piece) {
+            tc::TmemLoad16(base + (mb * kBufferColumns) + (piece * 16), ca);
+            tc::TmemLoadWait16(ca);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              acc2[(piece * 8) + i] =
+                  Add2(Pack2(__uint_as_float(ca[2 * i]), __uint_as_float(ca[(2 * i) + 1])), acc2[(piece * 8) + i]);
             }
           }
-        }
-        const std::uint64_t bx2 = Pack2(bx, bx);
-#pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          const float4 x4 = ax4[v];  // the same address in every lane: a broadcast
-          // (ax * C) rounded, times d8, added: as the scalar sequence, two rows at once
-          const std::uint64_t u01 =
-              Mul2(Pack2(static_cast<float>(static_cast<int>(r[(4 * v)])),
-                         static_cast<float>(static_cast<int>(r[(4 * v) + 1]))),
-                   Pack2(x4.x, x4.y));
-          const std::uint64_t u23 =
-              Mul2(Pack2(static_cast<float>(static_cast<int>(r[(4 * v) + 2])),
-                         static_cast<float>(static_cast<int>(r[(4 * v) + 3]))),
-                   Pack2(x4.z, x4.w));
-          acc2[2 * v] = Fma2(u01, bx2, acc2[2 * v]);
-          acc2[(2 * v) + 1] = Fma2(u23, bx2, acc2[(2 * v) + 1]);
-        }
-        if (++bb == kBuffers) {
-          bb = 0;
-          parity ^= 1u;
+          tc::TcFenceBefore();
+          __syncwarp();
+          if (lane == 0) tc::MbarArrive(&sh->tmem_empty[mb]);
         }
       }
-      __syncwarp();
-      if (lane == 0 && ok) tc::MbarArrive(&sh->empty[s]);  // the stage's scales are consumed
-    }
-    // The min terms: sum over the groups of (-dmin * m) * s8, taken by the tensor core.
-    if (ok) {
-      if (lane == 0) ok = tc::MbarWait(&sh->min_full, 0);
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok && lane == 0) give_up();
-    }
-    float acc[kEpilogueRows];  // the min terms first, then plus the folded groups
-    if (ok) {
-      tc::TcFenceAfter();
-      std::uint32_t r[32];
-      tc::TmemLoad32(tmem + lane_base + kMinColumn + (rowgroup * kEpilogueRows), r);
-      tc::TmemLoadWait();
+      float acc[kEpilogueRows];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) acc[j] = __uint_as_float(r[j]);
-    }
+      for (int i = 0; i < kEpilogueRows / 2; ++i) Unpack2(acc2[i], acc[2 * i], acc[(2 * i) + 1]);
+      const int first = row0 + (rowgroup * kEpilogueRows);
+      if (p.glu_out != nullptr) {
+        // The thread's 64 rows are twice 16 gate rows then the 16 up rows of the same outputs: one
+        // Q8_1-MMQ group of 32 outputs, whose scale and sum are formed exactly as the quantizer
+        // kernel does (eight lanes of four values, xor tree 4, 2, 1).
+        if (ok && col < c_end && first < a.nrows) {
+          float h[32], part[8], amax = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kEpilogueRows / 2; ++i) {
-      float lo, hi;
-      Unpack2(acc2[i], lo, hi);
-      acc[2 * i] += lo;
-      acc[(2 * i) + 1] += hi;
-    }
-    if (p.glu_out != nullptr) {
-      // The thread's 32 rows are 16 gate rows then the 16 up rows of the same outputs.  A
-      // Q8_1-MMQ group is 32 outputs: this thread's 16 and those of the thread of the same
-      // token one row group over (another warp), so the two trade their maxima and their
-      // four-value partial sums through shared memory (the first weight stage: every MMA has
-      // retired) and each forms the group's scale and sum exactly as the quantizer kernel
-      // does (eight lanes of four values, xor tree 4, 2, 1).  Every epilogue warp reaches the
-      // barrier, also one whose wait ran out: it stores nothing.
-      float h[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) h[j] = Glu(p.glu, acc[j], acc[16 + j], p.limit);
-      float part[4], amax = 0.0f;
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        part[l] = ((h[4 * l] + h[(4 * l) + 1]) + h[(4 * l) + 2]) + h[(4 * l) + 3];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) amax = fmaxf(amax, fabsf(h[(4 * l) + c]));
-      }
-      float* trade = reinterpret_cast<float*>(w_tiles);  // [4 row groups][128 tokens][8]
-      float* mine = trade + (((rowgroup * kTileCols) + tt) * 8);
-      mine[0] = amax;
-      mine[1] = ok ? 1.0f : 0.0f;
-      *reinterpret_cast<float4*>(mine + 4) = make_float4(part[0], part[1], part[2], part[3]);
-      asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
-      const float* other = trade + ((((rowgroup ^ 1) * kTileCols) + tt) * 8);
-      const float4 theirs = *reinterpret_cast<const float4*>(other + 4);
-      const bool both = ok && other[1] != 0.0f;
-      amax = fmaxf(amax, other[0]);
-      // lanes 0..3 of the quantizer hold the lower row group's values, 4..7 the upper's
-      const bool low = (rowgroup & 1) == 0;
-      const float p0 = low ? part[0] : theirs.x, p1 = low ? part[1] : theirs.y;
-      const float p2 = low ? part[2] : theirs.z, p3 = low ? part[3] : theirs.w;
-      const float p4 = low ? theirs.x : part[0], p5 = low ? theirs.y : part[1];
-      const float p6 = low ? theirs.z : part[2], p7 = low ? theirs.w : part[3];
-      const float sum = ((p0 + p4) + (p2 + p6)) + ((p1 + p5) + (p3 + p7));
-      const int out_first = (row0 / 2) + (rowgroup * 16);  // this thread's first GLU output
-      if (both && col < c_end && row0 + (rowgroup * kEpilogueRows) < a.nrows) {
-        std::uint32_t packed[4] = {0, 0, 0, 0};
-        float d = 0.0f;
-        if (amax > 0.0f) {
-          const float d_inv = 127.0f / amax;
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int q = static_cast<int>(roundf(h[j] * d_inv));
-            packed[j >> 2] |= (static_cast<std::uint32_t>(q) & 0xffu) << (8 * (j & 3));
+          for (int j = 0; j < 32; ++j) {
+            const int gate = ((j >> 4) * 32) + (j & 15);
+            h[j] = Glu(p.glu, acc[gate], acc[gate + 16], p.limit);
+            amax = fmaxf(amax, fabsf(h[j]));
           }
-          d = 1.0f / d_inv;
-        }
-        std::uint8_t* block = p.glu_out + (((static_cast<std::size_t>(out_first >> 7) * a.ncols) + col) * 144);
-        const int at = out_first & 127;
-        *reinterpret_cast<uint4*>(block + 16 + at) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        if (low) {
+#pragma unroll
+          for (int l = 0; l < 8; ++l) {
+            part[l] = ((h[4 * l] + h[(4 * l) + 1]) + h[(4 * l) + 2]) + h[(4 * l) + 3];
+          }
+          const float sum = ((part[0] + part[4]) + (part[2] + part[6])) +
+                            ((part[1] + part[5]) + (part[3] + part[7]));
+          std::uint32_t packed[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+          float d = 0.0f;
+          if (amax > 0.0f) {
+            const float d_inv = 127.0f / amax;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const int q = static_cast<int>(roundf(h[j] * d_inv));
+              packed[j >> 2] |= (static_cast<std::uint32_t>(q) & 0xffu) << (8 * (j & 3));
+            }
+            d = 1.0f / d_inv;
+          }
+          const int out_first = first / 2;  // this thread's first GLU output
+          std::uint8_t* block = p.glu_out + (((static_cast<std::size_t>(out_first >> 7) * a.ncols) + col) * 144);
+          const int at = out_first & 127;
+          auto* codes = reinterpret_cast<uint4*>(block + 16 + at);
+          codes[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+          codes[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
           *reinterpret_cast<std::uint32_t*>(block + ((at >> 5) * 4)) =
               static_cast<std::uint32_t>(__half_as_ushort(__float2half_rn(d))) |
               (static_cast<std::uint32_t>(__half_as_ushort(__float2half_rn(sum))) << 16);
         }
-      }
-    } else if (ok && col < c_end) {
-      const int dst_col = a.ids_dst != nullptr ? a.ids_dst[col] : col;
-      const int first = row0 + (rowgroup * kEpilogueRows);
-      float* out = a.dst + (static_cast<std::size_t>(dst_col) * a.dst_col_stride) + first;
-      // 128 contiguous bytes a thread: 128-bit stores when the output allows them
-      const bool vector = (a.dst_col_stride % 4 == 0) &&
-                          (reinterpret_cast<std::uintptr_t>(a.dst) % 16 == 0) && first + 32 <= a.nrows;
-      if (vector) {
-#pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          reinterpret_cast<float4*>(out)[v] =
-              make_float4(acc[4 * v], acc[(4 * v) + 1], acc[(4 * v) + 2], acc[(4 * v) + 3]);
-        }
-      } else {
+      } else if (ok && col < c_end) {
+        const int dst_col = a.ids_dst != nullptr ? a.ids_dst[col] : col;
+        float* out = a.dst + (static_cast<std::size_t>(dst_col) * a.dst_col_stride) + first;
+        // 256 contiguous bytes a thread: 128-bit stores when the output allows them
+        const bool vector = (a.dst_col_stride % 4 == 0) &&
+                            (reinterpret_cast<std::uintptr_t>(a.dst) % 16 == 0);
 #pragma unroll  // fully: a dynamic index would put acc[] in local memory
-        for (int j = 0; j < 32; ++j) {
-          if (first + j < a.nrows) out[j] = acc[j];
+        for (int v = 0; v < kEpilogueRows / 4; ++v) {
+          if (vector && first + (4 * v) + 4 <= a.nrows) {
+            reinterpret_cast<float4*>(out)[v] =
+                make_float4(acc[4 * v], acc[(4 * v) + 1], acc[(4 * v) + 2], acc[(4 * v) + 3]);
+          } else {
+#pragma unroll
+            for (int j = 4 * v; j < (4 * v) + 4; ++j) {
+              if (first + j < a.nrows) out[j] = acc[j];
+            }
+          }
         }
       }
     }
@@ -951,33 +1090,37 @@ int LaunchMmq(const llmp_b200_mmq_desc& d, const std::int32_t* worklist, int max
   int device = -1;
   cudaGetDevice(&device);
   if (configured_device != device) {
-    cudaError_t e = cudaFuncSetAttribute(MmqQ4KKernel<false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    if (e == cudaSuccess) {
-      e = cudaFuncSetAttribute(MmqQ4KKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    }
+    const auto allow = [](const void* kernel, int bytes) {
+      return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    };
+    cudaError_t e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<false, false>), kSmem<false>);
+    if (e == cudaSuccess) e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<true, false>), kSmem<true>);
+    if (e == cudaSuccess) e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<false, true>), kSmem<false>);
+    if (e == cudaSuccess) e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<true, true>), kSmem<true>);
     if (e != cudaSuccess) return fail(Failed(e, "mmq attribute"));
     configured_device = device;
   }
-  dim3 grid(static_cast<unsigned>((d.nrows + kTileRows - 1) / kTileRows), 1, 1);
+  std::int64_t tiles = (d.nrows + kTileRows - 1) / kTileRows;
   if (worklist != nullptr) {
     if (max_tiles < 1) return fail(Reject("mmq: a worklist needs its capacity"));
-    grid.y = static_cast<unsigned>(max_tiles);
+    p.col_tiles = max_tiles;
   } else {
     const int max_cols = d.expert_bounds != nullptr ? d.max_cols_per_expert : d.ncols;
     if (max_cols < 1) return fail(Reject("mmq: max_cols_per_expert >= 1 with experts"));
-    grid.y = static_cast<unsigned>((max_cols + kTileCols - 1) / kTileCols);
-    grid.z = static_cast<unsigned>(experts);
+    p.col_tiles = (max_cols + kTileCols - 1) / kTileCols;
+    tiles *= experts;
   }
-  if (grid.y > 65535u) return fail(Reject("mmq: more column tiles than a grid holds"));
+  if (p.col_tiles > 65535) return fail(Reject("mmq: more column tiles than a grid holds"));
+  tiles *= p.col_tiles;
+  // A CTA an SM (its shared memory and all of the SM's tensor memory), persistent: the next tile's
+  // operands and first groups come in under a tile's write-back.
+  const dim3 grid(static_cast<unsigned>(std::min<std::int64_t>(tiles, SmCount())));
   auto* s = static_cast<cudaStream_t>(stream);
-  if (slab != nullptr) {
-    MmqQ4KKernel<true><<<grid, kThreads, kSmem, s>>>(map_y, map_w, map_h, map_mw, p);
-  } else {
-    MmqQ4KKernel<false><<<grid, kThreads, kSmem, s>>>(map_y, map_w, map_h, map_mw, p);
-  }
-  const cudaError_t e = cudaPeekAtLastError();
-  if (e != cudaSuccess) return Failed(cudaGetLastError(), "mmq launch");
+  const auto kernel = slab != nullptr ? (sums != nullptr ? &MmqQ4KKernel<true, true> : &MmqQ4KKernel<true, false>)
+                                      : (sums != nullptr ? &MmqQ4KKernel<false, true> : &MmqQ4KKernel<false, false>);
+  const cudaError_t e = LaunchPdl(kernel, grid, dim3(kThreads), slab != nullptr ? kSmem<true> : kSmem<false>, s,
+                                  map_y, map_w, map_h, map_mw, p);
+  if (e != cudaSuccess) return Failed(e, "mmq launch");
   return 0;
 }
 
