@@ -6,6 +6,7 @@
 #include "vecq_ranks.h"
 #include "vecq_rowlane.cuh"
 #include "vecq_rowmma.cuh"
+#include "vecq_routed.cuh"
 
 namespace llmp_b200 {
 namespace vecq {
@@ -305,6 +306,17 @@ int LaunchVecQ(int type, const llmp_b200_vecq_desc* desc, int variant, bool f32_
         break;                            // refused cleanly: the rule below
       }
       break;
+    }
+  }
+  // A routed batch: the kernel that streams each named expert once for up to eight pairs.  Up to
+  // four tokens seldom share an expert and keep the kernel below, as does variant -2, whose bits
+  // must not depend on the token count.
+  if (variant == -1 && type == LLMP_B200_TYPE_Q4_K && d.ids != nullptr && d.tokens >= kRoutedTokens &&
+      !f32_input && q8_dst == nullptr && fan == nullptr) {
+    RoutedPlan routed{};
+    if (PlanRouted(d, SmCount(), &routed)) {
+      const cudaError_t status = LaunchRouted(d, routed, static_cast<cudaStream_t>(stream));
+      return status == cudaSuccess ? 0 : Failed(status, "vecq routed launch");
     }
   }
   if (variant == -2) variant = -1;

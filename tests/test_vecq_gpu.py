@@ -209,6 +209,50 @@ def test_routed_experts_match_the_oracle(cuda, orc, tokens, glu):
         assert float(np.abs(out - want).max()) <= 4e-5 * float(np.abs(want).max())
 
 
+@pytest.mark.parametrize("tokens,used,experts,n,k,glu,pad,per_slot", [
+    (5, 1, 1, 1, 256, 0, 0, False),         # one row, one column a row, one expert with five pairs
+    (5, 2, 3, 17, 768, 1, 0, True),         # a tile and one row; passes of eight and two
+    (9, 2, 2, 33, 1024, 3, 1, False),       # rows with a gap between them: a copy a row
+    (128, 8, 16, 40, 512, 0, 0, True),      # the largest batch: eight passes an expert
+    (64, 8, 128, 768, 2048, 1, 0, False),   # the MoE config's products
+    (64, 8, 128, 520, 768, 0, 0, True),
+    (16, 4, 1000, 48, 5120, 0, 0, False)])  # more columns than a group's warps
+def test_routed_batches_match_the_oracle(cuda, orc, tokens, used, experts, n, k, glu, pad, per_slot):
+    """The kernel that a routed batch takes, at the edges of its tiles, passes and rings; a pair
+    gives the same bits in another company and at another place among the pairs."""
+    torch = cuda
+    ops = _ops()
+    rng = np.random.default_rng(tokens * 31 + n + k)
+    row = k // 256 + pad
+    w = synth.q4_k_weights(rng, experts * n, row * 256).reshape(experts, n, -1)
+    g = synth.q4_k_weights(rng, experts * n, row * 256).reshape(experts, n, -1) if glu else None
+    ids = np.stack([rng.permutation(max(experts, used))[:used] % experts for _ in range(tokens)]).astype(np.int32)
+    ids[tokens // 2:, 0] = ids[0, 0]                 # a crowded expert
+    x = rng.normal(0, 1, size=(tokens * (used if per_slot else 1), k)).astype(np.float32)
+    q8 = ops.quantize_q8(to_dev(torch, x))
+    wd, gd = to_dev(torch, w), None if g is None else to_dev(torch, g)
+
+    def product(rows, blocks):
+        out = ops.vecq(wd, orc.Q4_K, k, n, blocks.contiguous(), len(rows), ids=to_dev(torch, ids[rows]), gate=gd,
+                       glu=glu, per_slot=per_slot, stride_row=row, stride_expert=n * row)
+        torch.cuda.synchronize()
+        assert ops.device_faults() == 0
+        return out
+
+    out = product(np.arange(tokens), q8)
+    rb = orc.q8_row_blocks(k)
+    f32, s64, a64 = orc.vecq(orc.Q4_K, w, q8.cpu().numpy(), k, n, tokens, ids=ids, used=used, stride_row=row,
+                             stride_expert=n * row, y_token=rb * used if per_slot else rb, y_slot=rb if per_slot else 0,
+                             g=g, glu=glu, want64=True)
+    if glu == 0:
+        assert_close_to_f64(out.cpu().numpy(), f32, s64, a64)
+    else:
+        assert float(np.abs(out.cpu().numpy() - f32).max()) <= 4e-5 * float(np.abs(f32).max())
+    rows = np.arange(tokens)[::-1][:max(5, tokens - 3)].copy()
+    other = product(rows, q8.view(tokens, -1)[torch.from_numpy(rows).cuda()])
+    assert torch.equal(other, out[torch.from_numpy(rows).cuda()])
+
+
 def test_routed_per_slot_activations_and_grouped_matrices(cuda, orc):
     torch = cuda
     ops = _ops()
