@@ -308,11 +308,13 @@ int LaunchVecQ(int type, const llmp_b200_vecq_desc* desc, int variant, bool f32_
       break;
     }
   }
-  // A routed batch: the kernel that streams each named expert once for up to eight pairs.  Up to
-  // four tokens seldom share an expert and keep the kernel below, as does variant -2, whose bits
-  // must not depend on the token count.
-  if (variant == -1 && type == LLMP_B200_TYPE_Q4_K && d.ids != nullptr && d.tokens >= kRoutedTokens &&
-      !f32_input && q8_dst == nullptr && fan == nullptr) {
+  // A routed batch: the kernel that streams each named expert once for up to eight pairs.  Fewer
+  // pairs seldom share an expert and keep the kernel below (a whole block of 128 experts, top 8,
+  // 2048 x 768, in us, that kernel first: 48.9 against 51.7 at 40 pairs, 67.2 / 67.9 at 64, 110.9 /
+  // 93.9 at 128, 452.7 / 166.9 at 768; 16 experts, top 2, 1024 x 512: 22.9 / 23.6 at 32, 26.9 / 25.2
+  // at 64), as does variant -2, whose bits must not depend on the token count.
+  if (variant == -1 && type == LLMP_B200_TYPE_Q4_K && d.ids != nullptr &&
+      d.tokens * d.used >= kRoutedFewest && !f32_input && q8_dst == nullptr && fan == nullptr) {
     RoutedPlan routed{};
     if (PlanRouted(d, SmCount(), &routed)) {
       const cudaError_t status = LaunchRouted(d, routed, static_cast<cudaStream_t>(stream));

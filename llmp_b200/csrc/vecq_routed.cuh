@@ -1,4 +1,4 @@
-// Routed Q4_K llmp.vecq for a batch of tokens (5 to 128): every expert that a token names is
+// Routed Q4_K llmp.vecq for a batch of tokens (72 pairs and more): every expert that a token names is
 // streamed once for up to eight of the (token, slot) pairs that name it, the int8 products on
 // the tensor cores (mma.sync m16n8k32, u8 x s8 -> s32) with the MMA's eight columns the pairs.
 // Interface and sums' contract are the reference's (src/kernels/ggml/vecq.h:23-49,
@@ -32,7 +32,7 @@
 namespace llmp_b200 {
 namespace vecq {
 
-constexpr int kRoutedTokens = 5;        // from here a batch takes this kernel
+constexpr int kRoutedFewest = 72;       // pairs from which a batch takes this kernel
 constexpr int kRoutedWarps = 16;        // 128 registers a thread
 constexpr int kRoutedPairs = kUnitTokens;  // pairs a pass
 constexpr int kRoutedTile = 16;         // rows a tile

@@ -1,4 +1,4 @@
-// The unit of the token-column kernels: 16 weight rows x one
+// The unit of the routed batch kernel (vecq_routed.cuh): 16 weight rows x one
 // Q4_K super-block x eight activation rows ("tokens"), a warp's work between two waits.
 //
 //   * The integer products: mma.sync m16n8k32 (u8 x s8 -> s32), one a 32-value sub-block, the
@@ -15,7 +15,8 @@
 // to them: sc * dot lands in a float by ONE integer multiply-add with the bits of 1.5 * 2^23
 // (|sc * dot| < 2^22; not so for the odd sub-blocks, whose dots are 16 times too large) and the
 // minima by one byte permute under 2^23's exponent, each less its constant by an exact F32 add; a
-// byte is one permute.  About 105 ALU instructions a unit.  (The minima as a BF16 contraction on
+// byte is one permute.  About 105 ALU instructions a unit (which by itself changed little: a tile's
+// latency, not its issue slots, is what the kernel waits for).  (The minima as a BF16 contraction on
 // the tensor core, d8 * sum q in three exact pieces: fewer instructions still, but its sums are off
 // by a quarter more.)
 #ifndef LLMP_B200_CSRC_VECQ_UNIT_CUH_
