@@ -295,9 +295,11 @@ int LaunchVecQ(int type, const llmp_b200_vecq_desc* desc, int variant, bool f32_
   // plan's whatever the token count (what llmp_b200_mmvq_rows runs on).
   if (variant == -1 && type == LLMP_B200_TYPE_Q4_K && d.ids == nullptr && d.used == 1 &&
       d.tokens <= 8 && !f32_input && q8_dst == nullptr && d.stride_row == d.ncols_x / 256) {
+    bool ranked = false;
     for (int i = 0; i < kMeasuredRankCount; ++i) {
       const MeasuredRank& r = kMeasuredRanks[i];
       if (r.k != d.ncols_x || r.n != d.nrows || (r.glu != 0) != glu || r.tokens != p) continue;
+      ranked = true;
       for (int v = 0; v < kVariantCount; ++v) {
         if (std::strcmp(kVariants[v].name, r.variant) != 0) continue;
         if (v == kRowLaneVariant) break;  // the rule below is that kernel
@@ -306,6 +308,19 @@ int LaunchVecQ(int type, const llmp_b200_vecq_desc* desc, int variant, bool f32_
         break;                            // refused cleanly: the rule below
       }
       break;
+    }
+    // A product that the table does not have: the row-lane kernel's dot products go up with the
+    // passes' token count (2, 4, 8), the token-column MMAs' time hardly with it.  From five tokens
+    // those, two CTAs an SM for a GLU where they fit (us at 5 and 8 tokens, row-lane first: gate |
+    // up 1280 -> 3072 13.9, 14.6 against 5.7, 6.2; 3328 -> 6400 22.2, 22.9 / 14.4, 15.0; 4608 ->
+    // 9216, one CTA an SM, 36.4, 36.9 / 24.5, 24.6; down 3072 -> 1280 10.0, 11.0 / 4.7, 5.2; 9216 ->
+    // 4608 19.8, 20.9 / 12.3, 12.7), and for a GLU over short rows from three (at 3 tokens 1024 ->
+    // 4096 7.3 against 5.3, 1792 -> 13312 19.0 / 14.0; but 2304 -> 7680 11.3 / 11.9).
+    if (!ranked && d.tokens >= (glu && d.ncols_x < kTokenColumnsShortRow ? 3 : 5)) {
+      for (int v = kTokenColumnsVariant + (glu ? 1 : 0); v >= kTokenColumnsVariant; --v) {
+        const int status = LaunchVecQ(type, desc, v, false, nullptr, nullptr, nullptr, stream, fan);
+        if (status <= 0) return status;
+      }
     }
   }
   // A routed batch: the kernel that streams each named expert once for up to eight pairs.  Fewer

@@ -395,11 +395,24 @@ VecQRowMmaKernel(const Desc a, const RowMmaPlan plan) {
       float v[kMats];
 #pragma unroll
       for (int m = 0; m < kMats; ++m) {
-        float s = 0.0f;
-        for (int w = 0; w < plan.col_groups; ++w) {
-          s += partial[(((static_cast<std::size_t>(w) * plan.pass_pad + r) * P + p) * kMats) + m];
+        const auto at = [&](int w) {
+          return partial[(((static_cast<std::size_t>(w) * plan.pass_pad + r) * P + p) * kMats) + m];
+        };
+        if constexpr (kTokenColumns) {
+          // four chains: their loads and adds overlap, and a third of the roundings in a row
+          float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+          for (int w = 0; w < plan.col_groups; w += 4) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              if (w + i < plan.col_groups) s[i] += at(w + i);
+            }
+          }
+          v[m] = (s[0] + s[1]) + (s[2] + s[3]);
+        } else {
+          float s = 0.0f;
+          for (int w = 0; w < plan.col_groups; ++w) s += at(w);
+          v[m] = s;
         }
-        v[m] = s;
       }
       float* dst = a.dst + (static_cast<std::size_t>(p) * a.dst_token) + first + r;
       float result;

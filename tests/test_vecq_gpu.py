@@ -209,6 +209,35 @@ def test_routed_experts_match_the_oracle(cuda, orc, tokens, glu):
         assert float(np.abs(out - want).max()) <= 4e-5 * float(np.abs(want).max())
 
 
+@pytest.mark.parametrize("tokens,n,k,glu,same_as", [
+    (5, 17, 768, 0, "rowmma.t8"), (8, 1280, 3072, 0, "rowmma.t8"), (4, 1280, 3072, 0, "rowlane"),
+    (5, 40, 2304, 1, "rowmma.t8c2"), (4, 40, 2304, 1, "rowlane"), (3, 300, 1792, 1, "rowmma.t8c2"),
+    (2, 300, 1792, 1, "rowlane"), (8, 600, 13312, 0, "rowlane")])   # the last: eight tokens do not fit beside a tile
+def test_products_without_a_rank_row_take_the_rule(cuda, orc, tokens, n, k, glu, same_as):
+    """The rule by rows and tokens for products that the rank table does not have: the bits of the
+    kernel it names, and the oracle's sums."""
+    torch = cuda
+    ops = _ops()
+    assert not any(r["k"] == k and r["n"] == n for r in ops.vecq_ranks())
+    rng = np.random.default_rng(tokens + n + k)
+    w = synth.q4_k_weights(rng, n, k)
+    g = synth.q4_k_weights(rng, n, k) if glu else None
+    x = rng.normal(0, 1, size=(tokens, k)).astype(np.float32)
+    q8 = ops.quantize_q8(to_dev(torch, x))
+    wd, gd = to_dev(torch, w), None if g is None else to_dev(torch, g)
+    out = ops.vecq(wd, orc.Q4_K, k, n, q8, tokens, gate=gd, glu=glu)
+    named = ops.vecq(wd, orc.Q4_K, k, n, q8, tokens, gate=gd, glu=glu,
+                     variant=-2 if same_as == "rowlane" else ops.vecq_variants().index(same_as))
+    torch.cuda.synchronize()
+    assert ops.device_faults() == 0
+    assert torch.equal(out, named)
+    f32, s64, a64 = orc.vecq(orc.Q4_K, w, q8.cpu().numpy(), k, n, tokens, g=g, glu=glu, want64=True)
+    if glu == 0:
+        assert_close_to_f64(out.cpu().numpy(), f32[:, 0], s64[:, 0], a64[:, 0])
+    else:
+        assert float(np.abs(out.cpu().numpy() - f32[:, 0]).max()) <= 4e-5 * float(np.abs(f32).max())
+
+
 @pytest.mark.parametrize("tokens,used,experts,n,k,glu,pad,per_slot", [
     (75, 1, 1, 1, 256, 0, 0, False),        # one row, one column a row, one expert with every pair
     (39, 2, 3, 17, 768, 1, 0, True),        # a tile and one row; the fewest pairs; short last passes
