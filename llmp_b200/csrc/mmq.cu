@@ -380,7 +380,9 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
   unsigned char* raw = zeros + kScaleTileBytes;                        // [kRawStages] raw stages
   Shared* sh = reinterpret_cast<Shared*>(raw + (kRawStages * kRawBytes<kSlab>));
 
-  const int warp = static_cast<int>(threadIdx.x) >> 5;
+  // (the shuffles tell the compiler that these are the warp's: tensor-memory addresses then live in
+  // uniform registers)
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x) >> 5, 0);
   const int lane = static_cast<int>(threadIdx.x) & 31;
   const int ksteps = a.k / kBK;
   if ((tc::Smem(smem) & 1023u) != 0) {  // uniform: the tiles' layout needs it
@@ -452,7 +454,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
     return tile;  // nothing to do, for every role alike, when col0 >= c_end
   };
 
-  const std::uint32_t tmem = sh->tmem_base;
+  const std::uint32_t tmem = __shfl_sync(0xffffffffu, sh->tmem_base, 0);
   volatile std::uint32_t* abort_flag = &sh->abort;
   auto give_up = [&]() {
     *abort_flag = 1;
