@@ -798,6 +798,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
       const int col = tile.col0 + tt;  // this thread's sorted column
 #pragma unroll
       for (int j = 0; j < kEpilogueRows / 2; ++j) acc2[j] = 0ull;
+#pragma unroll 4  // a k-step: buffers and parities are constants (eight groups miss the instruction cache)
       for (int g = 0; g < groups; ++g) {
         const int b = static_cast<int>(turn % kBuffers);
         const std::uint32_t at = base + (b * kBufferColumns);
