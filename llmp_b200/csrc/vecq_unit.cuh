@@ -22,6 +22,8 @@
 #ifndef LLMP_B200_CSRC_VECQ_UNIT_CUH_
 #define LLMP_B200_CSRC_VECQ_UNIT_CUH_
 
+#include <cfloat>
+
 #include "vecq_rowmma.cuh"
 
 namespace llmp_b200 {
@@ -99,6 +101,11 @@ struct Index {
   static constexpr int value = i;
 };
 
+// The rounding of a sum or product that is infinite comes out as inf - inf: a number in its place,
+// and the infinity it is added to stands.  (One instruction, where a test of the sum is two and a
+// register: the two-matrix kernel has none to spare.)
+__device__ __forceinline__ float Finite(float rounding) { return fmaxf(rounding, -FLT_MAX); }
+
 // sums[row g / g + 8][token 2t / 2t + 1] += the unit, for `mats` matrices whose blocks of rows g and
 // g + 8 start at lo[m] and hi[m]; c: the column among the staged ones.
 template <int kMats>
@@ -164,7 +171,7 @@ __device__ __forceinline__ void TokenUnit(const unsigned char* const (&lo)[kMats
         // d * p - dmin * q with one rounding of the two products
         const float p = pr[m][h][j][0] + pr[m][h][j][1], q = mr[m][h][j][0] + mr[m][h][j][1];
         const float main = d * p;
-        sums[m][h][j] += fmaf(dm, q, main) + fmaf(d, p, -main);
+        sums[m][h][j] += fmaf(dm, q, main) + Finite(fmaf(d, p, -main));
       }
     }
 }
@@ -192,7 +199,7 @@ __device__ __forceinline__ float SumColumns(const float* at, int columns, int st
   for (int i = 0; i < 3; ++i) {
     if (w + i < columns) add(at[(w + i) * stride]);
   }
-  return sum + rest;
+  return sum + Finite(rest);
 }
 
 }  // namespace vecq

@@ -282,6 +282,57 @@ def test_routed_batches_match_the_oracle(cuda, orc, tokens, used, experts, n, k,
     assert torch.equal(other, out[torch.from_numpy(rows).cuda()])
 
 
+@pytest.mark.parametrize("k,glu", [(256, 0), (1024, 0), (5120, 0), (768, 2), (2048, 2)])
+def test_routed_batches_keep_infinities(cuda, orc, k, glu):
+    """A block whose d or dmin is infinite gives the oracle's signed infinity where its terms agree
+    and NaN only where they do not (with the clamped GLU, what the clamp makes of an infinite up
+    value); the other rows keep their bits."""
+    torch = cuda
+    ops = _ops()
+    rng = np.random.default_rng(k + glu)
+    tokens, used, experts, n, nb, limit = 40, 2, 3, 21, k // 256, 7.0
+
+    def weights():
+        w = synth.q4_k_weights(rng, experts * n, k).reshape(experts * n, nb, 144)
+        w[:, :, 4:16] = synth.pack_q4_k_scales(rng.integers(1, 64, size=(experts * n, nb, 8), dtype=np.uint8),
+                                               rng.integers(1, 64, size=(experts * n, nb, 8), dtype=np.uint8))
+        w[:, :, 16:] |= 0x11                     # codes of 1 and more: with positive inputs no sum is zero
+        return w.reshape(experts, n, nb, 144)
+
+    clean, g = weights(), weights() if glu else None
+    if glu:
+        g[..., 2:4] = 0                          # gates of no minima: positive, so silu does not hide the up value
+    w = clean.copy()
+    inf = np.array([np.inf], np.float16).view(np.uint8)
+    planted = {1: [(0, 0, inf)], 2: [(nb - 1, 2, inf)], 3: [(nb // 2, 0, inf ^ np.uint8([0, 0x80]))],
+               5: [(0, 0, inf), (0, 2, inf)], 7: [(0, 0, inf), (nb - 1, 2, inf)], 20: [(nb - 1, 0, inf)]}
+    for row, places in planted.items():
+        for block, at, bits in places:
+            w[0, row, block, at:at + 2] = bits
+    ids = np.stack([rng.permutation(experts)[:used] for _ in range(tokens)]).astype(np.int32)
+    x = (np.abs(rng.normal(0, 1, size=(tokens, k))) + 0.1).astype(np.float32)
+    q8 = ops.quantize_q8(to_dev(torch, x))
+
+    def product(weight):
+        return ops.vecq(to_dev(torch, weight.reshape(experts, n, -1)), orc.Q4_K, k, n, q8, tokens, ids=to_dev(torch, ids),
+                        gate=None if g is None else to_dev(torch, g.reshape(experts, n, -1)), glu=glu,
+                        limit=limit if glu else 0.0, stride_expert=n * nb).cpu().numpy()
+
+    out, plain = product(w), product(clean)
+    want = orc.vecq(orc.Q4_K, w.reshape(experts, n, -1), q8.cpu().numpy(), k, n, tokens, ids=ids, used=used,
+                    stride_expert=n * nb, g=None if g is None else g.reshape(experts, n, -1), glu=glu,
+                    limit=limit if glu else 0.0)
+    hit = (ids == 0)[:, :, None] & np.isin(np.arange(n), list(planted))
+    assert hit.any() and np.array_equal(out[~hit], plain[~hit])
+    if glu == 0:
+        assert np.isposinf(want[hit]).any() and np.isneginf(want[hit]).any() and np.isnan(want[hit]).any()
+        assert np.array_equal(out[hit], want[hit], equal_nan=True)
+    else:
+        # an up of +-limit times silu of a finite gate, the gate's F32 sum the oracle's to 1e-5 of its scale
+        assert np.isfinite(want).all() and (want[hit] < -1).any() and (want[hit] > 1).any()
+        assert float(np.abs(out - want).max()) <= 4e-5 * float(np.abs(want).max())
+
+
 def test_routed_per_slot_activations_and_grouped_matrices(cuda, orc):
     torch = cuda
     ops = _ops()
