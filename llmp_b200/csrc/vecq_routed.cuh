@@ -23,7 +23,8 @@
 //     exact.
 //   * A pair's result does not depend on its company or on its place among the pairs.
 //   * Every mbarrier wait is bounded and reports through the fault counter; nothing of a tile
-//     that did not land is stored.
+//     that did not land is stored, and the group that waited for it requests no more and waits
+//     (bounded again) for what it has in flight before the CTA may end.
 #ifndef LLMP_B200_CSRC_VECQ_ROUTED_CUH_
 #define LLMP_B200_CSRC_VECQ_ROUTED_CUH_
 
@@ -209,8 +210,9 @@ VecQRoutedKernel(const Desc a, const RoutedPlan plan) {
     want_tile = static_cast<int>(want % plan.tiles);
     want_expert = find(want_pass);
   }
+  long want_end = u1;  // nothing more is requested once a wait has run out
   const auto request = [&]() {
-    if (want >= u1) return;
+    if (want >= want_end) return;
     const int r0 = want_tile * kRoutedTile;
     const int n = min(kRoutedTile, a.nrows - r0);
     std::uint64_t* bar = &full[(group * plan.stages) + want_stage];
@@ -283,6 +285,7 @@ VecQRoutedKernel(const Desc a, const RoutedPlan plan) {
         atomicAdd(plan.faults, 1u);
       }
       healthy = __shfl_sync(0xffffffffu, healthy ? 1 : 0, 0) != 0;
+      if (!healthy) want_end = 0;
       const unsigned char* rows_at = ring + (static_cast<std::size_t>(stage) * stage_bytes);
       // rows g and g + 8 of the tile, clamped into the matrix (the last tile may be short)
       const unsigned char* lo_at = rows_at + (min(g, rows - 1) * plan.pitch);
@@ -348,6 +351,15 @@ VecQRoutedKernel(const Desc a, const RoutedPlan plan) {
       }
     }
     u = end;
+  }
+  if (wc == 0 && !healthy) {
+    // what the group still has in flight must not outlive the CTA: its ring's last requests
+    const long first = (static_cast<long>(list->passes) * plan.tiles * blockIdx.x) / gridDim.x + group;
+    const long requested = (want - first) / plan.groups;
+    for (long i = max(0L, requested - plan.stages); i < requested; ++i) {
+      MbarWait(&full[(group * plan.stages) + static_cast<int>(i % plan.stages)],
+               static_cast<std::uint32_t>(i / plan.stages) & 1u);
+    }
   }
 }
 
