@@ -392,25 +392,43 @@ VecQRowMmaKernel(const Desc a, const RowMmaPlan plan) {
     for (int i = tid; i < count * P; i += static_cast<int>(blockDim.x)) {
       const int r = i / P, p = i % P;
       if (p >= a.tokens) continue;
+      const auto at = [&](int w) {
+        return partial + (((static_cast<std::size_t>(w) * plan.pass_pad + r) * P + p) * kMats);
+      };
       float v[kMats];
-#pragma unroll
-      for (int m = 0; m < kMats; ++m) {
-        const auto at = [&](int w) {
-          return partial[(((static_cast<std::size_t>(w) * plan.pass_pad + r) * P + p) * kMats) + m];
-        };
-        if constexpr (kTokenColumns) {
-          // four chains: their loads and adds overlap, and a third of the roundings in a row
-          float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-          for (int w = 0; w < plan.col_groups; w += 4) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              if (w + i < plan.col_groups) s[i] += at(w + i);
-            }
+      if constexpr (kTokenColumns) {
+        // Four chains, a quarter of the roundings in a row: the sums' error stays below the row-lane
+        // kernel's, whose products the launch rule gives to this one (3072 -> 1280 at 8 tokens 9.3e-8
+        // against 9.5e-8 off the double product; one chain 1.0e-7).  Whole fours without a test a
+        // column, and both matrices' sums in one load: with a test each and one matrix after the
+        // other a step of 34 feed-forward blocks took 949 us at 3 tokens and 1066 at 8, and takes 930
+        // and 1055 so (one chain: 939 and 1057); gate | up 2560 -> 10240 at 8 tokens 15.50 -> 15.26.
+        float s[4][kMats] = {};
+        const auto add = [&](int chain, int w) {
+          if constexpr (kGlu) {
+            const float2 q = *reinterpret_cast<const float2*>(at(w));
+            s[chain][0] += q.x;
+            s[chain][1] += q.y;
+          } else {
+            s[chain][0] += *at(w);
           }
-          v[m] = (s[0] + s[1]) + (s[2] + s[3]);
-        } else {
+        };
+        int w = 0;
+        for (; w + 4 <= plan.col_groups; w += 4) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) add(c, w + c);
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          if (w + c < plan.col_groups) add(c, w + c);
+        }
+#pragma unroll
+        for (int m = 0; m < kMats; ++m) v[m] = (s[0][m] + s[1][m]) + (s[2][m] + s[3][m]);
+      } else {
+#pragma unroll
+        for (int m = 0; m < kMats; ++m) {
           float s = 0.0f;
-          for (int w = 0; w < plan.col_groups; ++w) s += at(w);
+          for (int w = 0; w < plan.col_groups; ++w) s += at(w)[m];
           v[m] = s;
         }
       }
