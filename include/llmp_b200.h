@@ -121,11 +121,15 @@ typedef struct llmp_b200_vecq_desc {
  * CheckVecQ (src/kernels/ggml/llmp_ops.cc:2915-2982).  Types: Q8_0, Q4_K.
  * variant >= 0: that launch configuration (status > 0 if it does not take the product).
  * variant -1: the configuration that measured fastest on B200 for this very (k, n, GLU,
- * token count) when the rank table has it, else the rule for the shape; a token's F32 bits
- * may then differ between token counts (as the reference's MMVQ's do).
- * variant -2: the rule for the shape alone, whose geometry is the one-token plan's whatever
- * the token count: a token's bits do not depend on its company (the reference's
- * row_invariant capability; llmp_b200_mmvq_rows runs on it). */
+ * token count) when the rank table has it, else a rule by size: dense Q4_K products of 5 to 8
+ * tokens (of 3 to 8 with a GLU and k < 2048) take the token-column kernel, routed Q4_K products of
+ * 72 (token, slot) pairs and more the kernel that streams each named expert once, the others
+ * variant -2's.  These kernels add a row's super-blocks in different orders, so a token's F32 bits
+ * may differ between token counts and between numbers of pairs (as the reference's MMVQ's do
+ * between column counts).
+ * variant -2: one kernel for a shape, its geometry the one-token plan's whatever the token
+ * count: a token's bits do not depend on its company (the reference's row_invariant
+ * capability; llmp_b200_mmvq_rows runs on it). */
 int llmp_b200_vecq_variants(void);
 const char* llmp_b200_vecq_variant_name(int variant);
 int llmp_b200_vecq(int type, const llmp_b200_vecq_desc* desc, int variant, void* stream);
@@ -141,7 +145,8 @@ const char* llmp_b200_vecq_rank(int row, int* k, int* n, int* glu, int* tokens, 
  * :20-47, vecq.cu:1095-1175); here desc->y points at the F32 activations
  * themselves ([k, tokens], y_token FLOATS between tokens) and every CTA
  * quantizes them to Q8_1 in shared memory with the quantizer's arithmetic, so
- * the sums are the two-call path's bit for bit and one launch is saved.  Taken
+ * the sums are those of the quantizer and llmp_b200_vecq at variant -2 bit for
+ * bit (variant -1 may take another kernel) and one launch is saved.  Taken
  * for dense Q4_K products of up to 8 tokens (others: status > 0, use the two
  * calls).  q8_out (or NULL): receives the Q8_1 blocks of the first k / 32
  * blocks of each token's row, rows llmp_b200_q8_1_row_blocks(k) blocks apart. */
@@ -150,7 +155,7 @@ int llmp_b200_vecq_f32(int type, const llmp_b200_vecq_desc* desc, void* q8_out, 
 /* The product with the quantization of its OUTPUT fused: in the decode graph a
  * product's F32 result usually feeds the QuantizeQ8 node of the next product
  * (src/kernels/ggml/vecq.cu:1095-1111 after :1168; shared_q8.h:20-47).  This
- * entry writes desc->dst as llmp_b200_vecq does and, besides, the Q8_1 blocks of
+ * entry writes desc->dst as llmp_b200_vecq at variant -2 does and, besides, the Q8_1 blocks of
  * every token's output row into q8_dst ([tokens][nrows / 32] blocks of 36 bytes):
  * the warp that completes a 32-row block quantizes it with the quantizer's
  * arithmetic, so the blocks equal llmp_b200_q8_1_quantize(dst) bit for bit and

@@ -290,9 +290,10 @@ int LaunchVecQ(int type, const llmp_b200_vecq_desc* desc, int variant, bool f32_
   while (p > 1 && StageBytes(d.ncols_x, p) > 200 * 1024) p /= 2;
   // variant -1: the fastest measured configuration of this very product, when the table
   // has it (the bits of a token may then differ between token counts, as the reference's
-  // MMVQ's do); a configuration that turns the product down falls through to the rule
-  // below.  variant -2: the rule below alone, whose row-lane geometry is the one-token
-  // plan's whatever the token count (what llmp_b200_mmvq_rows runs on).
+  // MMVQ's do); a configuration that turns the product down falls through to the rules
+  // below.  variant -2: one kernel a shape (dense Q4_K: row-lane), whose geometry is the
+  // one-token plan's whatever the token count (what llmp_b200_mmvq_rows runs on; the fused
+  // forms' bits are its too).
   if (variant == -1 && type == LLMP_B200_TYPE_Q4_K && d.ids == nullptr && d.used == 1 &&
       d.tokens <= 8 && !f32_input && q8_dst == nullptr && d.stride_row == d.ncols_x / 256) {
     bool ranked = false;

@@ -211,8 +211,8 @@ def vecq_f32(weights: torch.Tensor, wtype: int, k: int, n: int, x: torch.Tensor,
              gate: torch.Tensor | None = None, glu: int = GLU_NONE, limit: float = 0.0,
              out: torch.Tensor | None = None, q8_out: torch.Tensor | None = None) -> torch.Tensor:
     """QuantizeQ8 + VecQ in one launch: x F32 [tokens <= 8, k] (rows 16-byte aligned), dense
-    Q4_K weights [n, k] -> F32 [tokens, n].  q8_out (uint8 [tokens, q8_1_row_blocks(k) * 36])
-    optionally receives the Q8_1 blocks the kernel formed."""
+    Q4_K weights [n, k] -> F32 [tokens, n], the bits of quantize_q8 and vecq(variant=-2).  q8_out
+    (uint8 [tokens, q8_1_row_blocks(k) * 36]) optionally receives the Q8_1 blocks the kernel formed."""
     _need(weights, torch.uint8, "vecq_f32 weights")
     _need(x, torch.float32, "vecq_f32 activations")
     if x.dim() != 2 or x.stride(1) != 1:
@@ -247,7 +247,8 @@ def vecq_q8(weights: torch.Tensor, wtype: int, k: int, n: int, q8: torch.Tensor,
             limit: float = 0.0, out: torch.Tensor | None = None,
             q8_dst: torch.Tensor | None = None):
     """VecQ + QuantizeQ8 of its output in one launch: dense Q4_K weights [n, k] (n a multiple
-    of 512), q8 of [tokens <= 8, k] -> (F32 [tokens, n], its Q8_1 blocks uint8 [tokens, n/32*36])."""
+    of 512), q8 of [tokens <= 8, k] -> (F32 [tokens, n], its Q8_1 blocks uint8 [tokens, n/32*36]);
+    the bits of vecq(variant=-2)."""
     _need(weights, torch.uint8, "vecq_q8 weights")
     _need(q8, torch.uint8, "vecq_q8 q8")
     _need(rows_done, torch.int32, "vecq_q8 counters")

@@ -384,7 +384,7 @@ def test_operands_the_kernels_do_not_take_are_refused_before_launch(cuda, orc):
 
 
 @pytest.mark.parametrize("n,k,tokens,glu", [(10240, 2560, 1, 3), (2560, 10240, 1, 0),
-                                            (333, 2560, 8, 1), (64, 512, 3, 0)])
+                                            (333, 2560, 8, 1), (64, 512, 3, 0), (1280, 3072, 8, 0)])
 def test_fused_quantization_gives_the_two_call_bits(cuda, orc, n, k, tokens, glu):
     """llmp_b200_vecq_f32 quantizes the F32 activations inside the product kernel: its Q8_1
     blocks are the quantizer's bit for bit, and so are the sums of the two-call path."""
@@ -411,7 +411,7 @@ def test_fused_quantization_gives_the_two_call_bits(cuda, orc, n, k, tokens, glu
 
 @pytest.mark.parametrize("n,k,tokens,glu", [(10240, 2560, 1, 3), (2560, 10240, 1, 0),
                                             (2560, 10240, 8, 0), (1024, 512, 3, 1),
-                                            (512, 256, 2, 0)])
+                                            (512, 256, 2, 0), (1024, 3072, 8, 0)])
 def test_fused_output_quantization_gives_the_two_call_bits(cuda, orc, n, k, tokens, glu):
     """llmp_b200_vecq_q8 also writes its output as Q8_1 blocks: the F32 output is the plain
     product's and the blocks are the quantizer's over that output, bit for bit; the row
