@@ -84,6 +84,44 @@ def test_dense_mmq_matches_the_oracle(cuda, orc, cols, n, k, mode):
     assert nmse <= 5e-4, nmse
 
 
+@pytest.mark.parametrize("mode", ["raw", "scratch", "slab"])
+@pytest.mark.parametrize("cols,n,k", [(130, 9473, 1280),    # 150 tiles of one section of min terms
+                                      (203, 10241, 2304),   # 162 of two, a partial second one
+                                      (203, 10241, 4352)])  # ... of three: an odd number, over both tiles of min operands
+def test_ctas_that_take_several_tiles(cuda, orc, cols, n, k, mode):
+    """More tiles than SMs: what a CTA carries from a tile to its next (stages, parities, the turn
+    of the tensor-memory buffers and of the min operands) changes no bit of what products of
+    fewer tiles than SMs give, exact group sums included; the last rows against the oracle."""
+    torch = cuda
+    ops = _ops()
+    tiles = lambda rows: (rows + 127) // 128 * ((cols + 127) // 128)  # noqa: E731
+    half = 128 * (n // 256)
+    assert tiles(half) <= ops.sm_count() and tiles(n - half) <= ops.sm_count() < tiles(n)
+    rng = np.random.default_rng(cols + n + k)
+    w = synth.q4_k_weights(rng, n, k)
+    yq = ops.mmq_quantize(to_dev(torch, rng.normal(0, 1, size=(cols, k)).astype(np.float32)))
+    wd = to_dev(torch, w)
+
+    def product(rows, call):
+        if mode == "scratch":
+            return call(rows, yq, k, rows.shape[0], scratch=ops.mmq_scratch(k, rows.shape[0]))
+        if mode == "slab":
+            return call(None, yq, k, rows.shape[0], slab=ops.q4k_relayout(rows, k, rows.shape[0]))
+        return call(rows, yq, k, rows.shape[0])
+
+    out, lo, hi = (product(rows, ops.mmq) for rows in (wd, wd[:half], wd[half:]))
+    assert torch.equal(out[:, :half], lo) and torch.equal(out[:, half:], hi)
+    if k == 1280:
+        same, sums = product(wd, ops.mmq_block_sums)
+        assert torch.equal(same, out)
+        assert torch.equal(sums[:, :half], product(wd[:half], ops.mmq_block_sums)[1])
+        assert torch.equal(sums[:, half:], product(wd[half:], ops.mmq_block_sums)[1])
+    torch.cuda.synchronize()
+    assert ops.device_faults() == 0
+    want32, want64 = orc.mmq_q4_k(w[-130:], yq.cpu().numpy(), k, 130, want64=True)
+    _check(out[:, -130:].cpu().numpy(), want32, want64)
+
+
 def test_routed_mmq_over_expert_sorted_columns(cuda, orc):
     """mul_mat_id: experts' weight matrices over the sorted (token, slot) columns,
     scattered back through ids_dst (src/kernels/ggml/mul_mat_q.cu:551-737)."""
@@ -195,7 +233,8 @@ def test_routed_mmq_takes_a_slab_of_experts(cuda, orc):
     _check(slab.cpu().numpy(), want32, want64)
 
 
-@pytest.mark.parametrize("cols,inter,k,glu", [(200, 256, 512, 1), (513, 768, 2048, 1), (64, 128, 256, 3)])
+@pytest.mark.parametrize("cols,inter,k,glu", [(200, 256, 512, 1), (513, 768, 2048, 1), (64, 128, 256, 3),
+                                              (203, 5120, 1280, 1)])   # more tiles than SMs
 def test_glu_write_back_equals_the_product_then_the_glu_quantizer(cuda, cols, inter, k, glu):
     """MulMatQGlu: the GLU and the requantization inside the gate | up product's write-back give,
     bit for bit, the blocks llmp_b200_moe_glu_quantize makes of the F32 product."""
