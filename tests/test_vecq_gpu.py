@@ -241,7 +241,9 @@ def test_products_without_a_rank_row_take_the_rule(cuda, orc, tokens, n, k, glu,
 @pytest.mark.parametrize("tokens,used,experts,n,k,glu,pad,per_slot", [
     (75, 1, 1, 1, 256, 0, 0, False),        # one row, one column a row, one expert with every pair
     (39, 2, 3, 17, 768, 1, 0, True),        # a tile and one row; the fewest pairs; short last passes
-    (43, 2, 2, 33, 1024, 3, 1, False),      # rows with a gap between them: a copy a row
+    (43, 2, 2, 33, 1024, 3, 1, False),      # a ring of two-matrix tiles that does not fit: the kernel of fewer pairs
+    (43, 2, 2, 33, 1280, 3, 1, False),      # rows with a gap between them: a copy a row
+    (43, 2, 2, 33, 1024, 0, 1, False),
     (128, 8, 16, 40, 512, 0, 0, True),      # the largest batch: eight passes an expert
     (64, 8, 128, 768, 2048, 1, 0, False),   # the MoE config's products
     (64, 8, 128, 520, 768, 0, 0, True),
@@ -261,14 +263,16 @@ def test_routed_batches_match_the_oracle(cuda, orc, tokens, used, experts, n, k,
     q8 = ops.quantize_q8(to_dev(torch, x))
     wd, gd = to_dev(torch, w), None if g is None else to_dev(torch, g)
 
-    def product(rows, blocks):
+    def product(rows, blocks, variant=-1):
         out = ops.vecq(wd, orc.Q4_K, k, n, blocks.contiguous(), len(rows), ids=to_dev(torch, ids[rows]), gate=gd,
-                       glu=glu, per_slot=per_slot, stride_row=row, stride_expert=n * row)
+                       glu=glu, per_slot=per_slot, stride_row=row, stride_expert=n * row, variant=variant)
         torch.cuda.synchronize()
         assert ops.device_faults() == 0
         return out
 
     out = product(np.arange(tokens), q8)
+    # variant -2 is the kernel of fewer pairs, which adds a row up in another order
+    assert torch.equal(out, product(np.arange(tokens), q8, variant=-2)) == (glu != 0 and k == 1024)
     rb = orc.q8_row_blocks(k)
     f32, s64, a64 = orc.vecq(orc.Q4_K, w, q8.cpu().numpy(), k, n, tokens, ids=ids, used=used, stride_row=row,
                              stride_expert=n * row, y_token=rb * used if per_slot else rb, y_slot=rb if per_slot else 0,
