@@ -4,9 +4,11 @@
 // Interface and sums' contract are the reference's (src/kernels/ggml/vecq.h:23-49,
 // vecq.cu:457-665); the ownership of an expert (vecq.cu:514-546) is by a list here.
 //
-// What bounds it: the named experts' bytes (HBM), then the fold's instruction stream, about 280
-// warp instructions a 16-row x 256-value unit, 37 us of issue slots for 128 experts of 2048 x
-// 768.  The register-staged kernel (vecq_impl.cuh) launches a grid row for every (token, slot)
+// What bounds it: a tile's latency.  A block of 128 experts, top 8, 2048 x 768 at 64 tokens takes
+// 147 us; its products' weights are 52 us of the measured copy rate and their instructions 64 us of
+// issue slots (443 and 554 warp instructions a 16-row x 256-value unit of gate | up and down, the
+// lists, the staging and the meetings counted), and of a warp's time between two instructions 41
+// and 30 % goes to the group's barrier.  The register-staged kernel (vecq_impl.cuh) launches a grid row for every (token, slot)
 // pair, most of which leave after scanning the ids, and its dot products take an instruction for
 // four values of ONE pair.
 //
@@ -268,14 +270,14 @@ VecQRoutedKernel(const Desc a, const RoutedPlan plan) {
     for (int i = tid; i < live * blocks; i += threads) {
       const int p = i / blocks, b = i - (p * blocks);
       const int pr = pairs[p];
-      StageUnitBlock(acts, layout, kRoutedPairs, p, b,
+      StageUnitBlock(acts, layout, p, b,
                      static_cast<const std::uint8_t*>(a.y) +
                          ((static_cast<std::size_t>(pr >> 8) * a.y_token +
                            static_cast<std::size_t>(pr & 0xff) * a.y_slot + b) * 36));
     }
     __syncthreads();
 
-    const UnitLane at_lane(acts, layout, kRoutedPairs, live, lane);
+    const UnitLane at_lane(acts, layout, live, lane);
     for (; unit < end; unit += plan.groups, ++turn) {
       const int r0 = static_cast<int>(unit - first_unit) * kRoutedTile;
       const int rows = min(kRoutedTile, a.nrows - r0);
@@ -375,7 +377,7 @@ inline bool PlanRouted(const Desc& d, int sms, RoutedPlan* plan) {
   plan->tiles = (d.nrows + kRoutedTile - 1) / kRoutedTile;
   plan->packed = packed ? 1 : 0;
   plan->pitch = packed ? row_bytes : ((row_bytes + 127) / 128 * 128) + 32;
-  plan->acts_bytes = TokenActs(ur).Bytes(kRoutedPairs);
+  plan->acts_bytes = TokenActs(ur).Bytes();
   const int stage = mats * kRoutedTile * plan->pitch;
   const int fixed = plan->acts_bytes + static_cast<int>(sizeof(RoutedList)) + 128;
   const int limit = 225 * 1024;

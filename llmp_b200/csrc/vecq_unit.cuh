@@ -9,16 +9,15 @@
 //   * The fold: lane (g, t) holds rows g and g + 8 x tokens 2t and 2t + 1 and adds
 //     d8 * (sc * dot) and (d8 * sum q) * m, the even and the odd sub-blocks apart (half the
 //     roundings in a row).
-// The integer ALU takes two cycles a warp instruction on this part and the fold is mostly its work
-// (conversions, byte extracts, masks: 240 of 380 instructions as first written, per-opcode counts
-// of the 2560 -> 10240 gate | up product), while the multiply-add pipes idle.  So what can be goes
-// to them: sc * dot lands in a float by ONE integer multiply-add with the bits of 1.5 * 2^23
-// (|sc * dot| < 2^22; not so for the odd sub-blocks, whose dots are 16 times too large) and the
-// minima by one byte permute under 2^23's exponent, each less its constant by an exact F32 add; a
-// byte is one permute.  About 105 ALU instructions a unit (which by itself changed little: a tile's
-// latency, not its issue slots, is what the kernel waits for).  (The minima as a BF16 contraction on
-// the tensor core, d8 * sum q in three exact pieces: fewer instructions still, but its sums are off
-// by a quarter more.)
+// The integer ALU takes two cycles a warp instruction on this part, and the fold as the dense
+// token-column kernel writes it is mostly its work (conversions, byte extracts, masks) beside idle
+// multiply-add pipes.  So what can be goes to them: sc * dot lands in a float by ONE integer
+// multiply-add with the bits of 1.5 * 2^23 (|sc * dot| < 2^22; not so for the odd sub-blocks, whose
+// dots are 16 times too large) and the minima by one byte permute under 2^23's exponent, each less
+// its constant by an exact F32 add; a byte is one permute.  The ALU pipe is then busy 34 % of the
+// time and the multiply-add pipes 19 % (a tile's latency, not its issue slots, is what the kernel
+// waits for).  (The minima as a BF16 contraction on the tensor core, d8 * sum q in three exact
+// pieces: fewer instructions still, but its sums are off by a quarter more.)
 #ifndef LLMP_B200_CSRC_VECQ_UNIT_CUH_
 #define LLMP_B200_CSRC_VECQ_UNIT_CUH_
 
@@ -42,15 +41,15 @@ struct TokenActs {
   __host__ __device__ constexpr int Pitch() const { return (columns * 256) + 64; }
   // the four pairs' scales are read together: 32 bytes modulo 128
   __host__ __device__ constexpr int PairPitch() const { return (columns * 128) + 32; }
-  __host__ __device__ constexpr int Scales(int tokens) const { return tokens * Pitch(); }
-  __host__ __device__ constexpr int Bytes(int tokens) const {
-    return ((Scales(tokens) + (4 * PairPitch())) + 127) / 128 * 128;
+  __host__ __device__ constexpr int Scales() const { return kUnitTokens * Pitch(); }
+  __host__ __device__ constexpr int Bytes() const {
+    return ((Scales() + (kUnitTokens / 2 * PairPitch())) + 127) / 128 * 128;
   }
 };
 
 // One Q8_1 block (sub-block b of the staged columns) of token p.
-__device__ __forceinline__ void StageUnitBlock(unsigned char* acts, TokenActs layout, int tokens, int p,
-                                               int b, const std::uint8_t* block) {
+__device__ __forceinline__ void StageUnitBlock(unsigned char* acts, TokenActs layout, int p, int b,
+                                               const std::uint8_t* block) {
   const auto* src = reinterpret_cast<const std::uint32_t*>(block);
   std::uint32_t v[8];
   int isum = 0;
@@ -64,7 +63,7 @@ __device__ __forceinline__ void StageUnitBlock(unsigned char* acts, TokenActs la
   auto* codes = reinterpret_cast<uint2*>(row + ((b >> 1) * 64) + ((b & 1) * 8));
 #pragma unroll
   for (int t = 0; t < 4; ++t) codes[2 * t] = make_uint2(v[2 * t], v[(2 * t) + 1]);
-  float* scales = reinterpret_cast<float*>(acts + layout.Scales(tokens) + ((p >> 1) * layout.PairPitch())) +
+  float* scales = reinterpret_cast<float*>(acts + layout.Scales() + ((p >> 1) * layout.PairPitch())) +
                   (4 * b) + (p & 1);
   scales[0] = (b & 1) != 0 ? d * 0.0625f : d;
   scales[2] = d * static_cast<float>(isum);
@@ -89,10 +88,10 @@ __device__ __forceinline__ int ByteInt(std::uint32_t w) {
 struct UnitLane {
   const unsigned char* codes;
   const unsigned char* scales;
-  __device__ __forceinline__ UnitLane(const unsigned char* acts, TokenActs layout, int tokens, int live, int lane) {
+  __device__ __forceinline__ UnitLane(const unsigned char* acts, TokenActs layout, int live, int lane) {
     const int g = lane >> 2, t = lane & 3;
     codes = acts + (min(g, live - 1) * layout.Pitch()) + (16 * t);
-    scales = acts + layout.Scales(tokens) + (t * layout.PairPitch());
+    scales = acts + layout.Scales() + (t * layout.PairPitch());
   }
 };
 
