@@ -8,9 +8,9 @@
 // 147 us; its products' weights are 52 us of the measured copy rate and their instructions 64 us of
 // issue slots (443 and 554 warp instructions a 16-row x 256-value unit of gate | up and down, the
 // lists, the staging and the meetings counted), and of a warp's time between two instructions 41
-// and 30 % goes to the group's barrier.  The register-staged kernel (vecq_impl.cuh) launches a grid row for every (token, slot)
-// pair, most of which leave after scanning the ids, and its dot products take an instruction for
-// four values of ONE pair.
+// and 30 % goes to the group's barrier.  The register-staged kernel (vecq_impl.cuh) launches a
+// grid row for every (token, slot) pair, most of which leave after scanning the ids, and its dot
+// products take an instruction for four values of ONE pair.
 //
 //   * One persistent CTA an SM.  It builds the list of distinct experts and their pairs in shared
 //     memory (a hash table for the counts, a warp's scan over the pairs in order for the list; every
