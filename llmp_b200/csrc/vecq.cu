@@ -313,10 +313,13 @@ int LaunchVecQ(int type, const llmp_b200_vecq_desc* desc, int variant, bool f32_
     // A product that the table does not have: the row-lane kernel's dot products go up with the
     // passes' token count (2, 4, 8), the token-column MMAs' time hardly with it.  From five tokens
     // those, two CTAs an SM for a GLU where they fit (us at 5 and 8 tokens, row-lane first: gate |
-    // up 1280 -> 3072 13.9, 14.6 against 5.7, 6.2; 3328 -> 6400 22.2, 22.9 / 14.4, 15.0; 4608 ->
-    // 9216, one CTA an SM, 36.4, 36.9 / 24.5, 24.6; down 3072 -> 1280 10.0, 11.0 / 4.7, 5.2; 9216 ->
-    // 4608 19.8, 20.9 / 12.3, 12.7), and for a GLU over short rows from three (at 3 tokens 1024 ->
-    // 4096 7.3 against 5.3, 1792 -> 13312 19.0 / 14.0; but 2304 -> 7680 11.3 / 11.9).
+    // up 1280 -> 3072 21.3, 22.1 against 5.5, 6.0; 3328 -> 6400 22.1, 23.0 / 14.1, 14.5; 4608 ->
+    // 9216, one CTA an SM, 36.3, 37.0 / 23.9, 24.4; down 3072 -> 1280 11.1, 12.1 / 4.7, 5.2; 9216 ->
+    // 4608 19.8, 20.9 / 12.5, 12.9), and for a GLU over short rows from three (at 3 tokens 1024 ->
+    // 4096 8.9 against 5.1, 1792 -> 13312 18.9 / 13.7; but 2304 -> 7680 11.3 / 11.6).  The line by k
+    // is on the safe side: with few rows a CTA they win at three and four tokens too (3072 -> 1280
+    // 6.4 against 4.3, gate | up 2048 -> 3584 8.0 / 6.2, 3840 -> 2048 8.6 / 6.7), with many hardly
+    // (9216 -> 4608 12.2 / 12.0); such products stay on row-lane.
     if (!ranked && d.tokens >= (glu && d.ncols_x < kTokenColumnsShortRow ? 3 : 5)) {
       for (int v = kTokenColumnsVariant + (glu ? 1 : 0); v >= kTokenColumnsVariant; --v) {
         const int status = LaunchVecQ(type, desc, v, false, nullptr, nullptr, nullptr, stream, fan);

@@ -28,8 +28,13 @@ __all__ = ["available", "sm_count", "device_faults", "device_faults_clear", "blo
 TYPE_Q4_0, TYPE_Q5_0, TYPE_Q5_K, TYPE_Q6_K, TYPE_IQ4_NL = 2, 6, 13, 14, 20   # GGML's type ids
 _BLOCK = {TYPE_Q8_0: (32, 34), TYPE_Q4_K: (256, 144), N.TYPE_Q8_1: (32, 36), TYPE_Q4_0: (32, 18),
           TYPE_Q5_0: (32, 22), TYPE_IQ4_NL: (32, 18), TYPE_Q5_K: (256, 176), TYPE_Q6_K: (256, 210)}
-# moe_ffn: up to this many tokens take the routed decode products (measured on B200 against the
-# grouped tensor-core GEMM for 128 experts, top-8, hidden 2048, intermediate 768).
+# moe_ffn: up to this many tokens take the routed decode products.  No longer where the two meet on
+# B200: whole blocks take (us, routed products first, then the grouped tensor-core GEMM over slabs)
+# 170 against 513 at 96 tokens, 207 / 519 at 128 and 408 / 525 at 256 for 128 experts, top-8, hidden
+# 2048, intermediate 768; 128 / 288 at 96 and 307 / 293 at 256 for 32 experts, top-4, 2048 x 1536;
+# 50 / 53 at 96 and 61 / 53 at 128 for 16 experts, top-2, 1024 x 512.  The line stays because the
+# two sides round the activations in different formats (Q8_1, Q8_1-MMQ): moving it changes results,
+# and which weights a program relays.  A call's `decode_tokens` sets it.
 DECODE_TOKENS = 96
 
 
@@ -665,8 +670,8 @@ def moe_ffn(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, gate_up: 
     experts = gate_up.shape[0]
     # Few tokens: the decode products (routed llmp.vecq), which stream each named expert's
     # weights once per call, in calls of at most 128 tokens and 1,024 (token, slot) pairs (the
-    # kernel's limits).  Up to DECODE_TOKENS tokens that beats the tensor-core GEMM, whose
-    # 128-row tiles are nearly empty when an expert sees a handful of rows.
+    # kernel's limits).  With a handful of rows an expert that beats the tensor-core GEMM, whose
+    # 128-row tiles are then nearly empty.
     chunk = min(128, max(1, 1024 // used))
     if tokens <= MOE_DECODE_TOKENS and (decode_tokens is None or decode_tokens > 0) and \
             x.dtype == torch.float32 and x.stride(-1) == 1 and moe_decode_fits(tokens, used, hidden, inter):
