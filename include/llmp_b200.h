@@ -298,6 +298,11 @@ int llmp_b200_vecq_block_sums(int type, const void* w, const void* y, int k, int
 int64_t llmp_b200_mmq_q8_1_bytes(int64_t k, int64_t cols);
 int llmp_b200_mmq_quantize(const void* x, int is_bf16, int64_t row_stride, int64_t k, int64_t cols,
                            const int32_t* ids_src, void* out, void* stream);
+/* The same blocks for routed rows, each token quantized once: x [k, tokens]; position (device, I32
+ * [tokens][used], as llmp_b200_moe_route leaves it) names token t's columns of out, ordered
+ * [k / 128][tokens * used]; a negative one is skipped, and a column no position names is not written. */
+int llmp_b200_mmq_quantize_slots(const void* x, int is_bf16, int64_t row_stride, int64_t k, int64_t tokens,
+                                 const int32_t* position, int used, void* out, void* stream);
 
 /* The operands GGML's mmq_args carry as the reference fills them
  * (src/kernels/ggml/mul_mat_q.cu:632-658). */

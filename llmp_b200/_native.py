@@ -160,6 +160,8 @@ SIGNATURES = {
     "llmp_b200_mmq_q8_1_bytes": (C.c_int64, [C.c_int64, C.c_int64]),
     "llmp_b200_mmq_quantize": (C.c_int, [C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_int64,
                                          C.c_void_p, C.c_void_p, C.c_void_p]),
+    "llmp_b200_mmq_quantize_slots": (C.c_int, [C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_int64,
+                                               C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
     "llmp_b200_mmq_scratch": (C.c_size_t, [C.POINTER(MmqDesc), C.c_int]),
     "llmp_b200_mmq": (C.c_int, [C.POINTER(MmqDesc), C.c_int, C.c_void_p]),
     "llmp_b200_mmq_block_sums": (C.c_int, [C.POINTER(MmqDesc), C.c_void_p, C.c_void_p]),

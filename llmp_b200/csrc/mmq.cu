@@ -65,65 +65,119 @@ using Desc = llmp_b200_mmq_desc;
 
 // ------------------------------------------------------------------ quantizer
 // block_q8_1_mmq, DS4 layout: 4 x (FP16 d, FP16 sum of the inputs), 128 int8.
-// Blocks ordered [k / 128][col].  Eight lanes a 32-value group, four values a
-// lane; the sum is taken four-per-lane then over the lanes 4, 2, 1 apart.
+// Blocks ordered [k / 128][col].  A warp takes 256 values of k of kCols columns, a lane eight of a
+// 32-value group: 16- or 32-byte loads, all columns' on their way together, and neighbouring columns'
+// blocks, neighbours in memory, by one warp.  (A thread four values of one column, with a 64-bit
+// division each, was bound by its instructions: 28.5 us for 4096 x 4096 BF16 values, 1.8 TB/s.)
+// The stored sum's order is four values in order, then parts 4, 2, 1 apart.
+// kSlots: column t is quantized once and its blocks go to every column position[t * used + j] >= 0
+// (a routed token's rows), where ids_src would have a column's input read and quantized `used` times.
 template <bool kBf16>
+__device__ __forceinline__ void Load8(const void* __restrict__ x, std::int64_t at, float (&v)[8]) {
+  if constexpr (kBf16) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(x) + at);
+    const std::uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[(2 * i) + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  } else {
+    const float4* from = reinterpret_cast<const float4*>(static_cast<const float*>(x) + at);
+    const float4 lo = from[0], hi = from[1];
+    v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
+    v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+  }
+}
+
+template <bool kBf16, int kCols, bool kSlots>
 __global__ void __launch_bounds__(256)
-QuantizeMmqKernel(const void* __restrict__ x, std::int64_t row_stride, int k, std::int64_t cols,
-                  const std::int32_t* __restrict__ ids_src, std::uint8_t* __restrict__ out,
-                  std::int64_t lanes_total) {
+QuantizeMmqKernel(const void* __restrict__ x, std::int64_t row_stride, int k, int cols,
+                  const std::int32_t* __restrict__ ids_src, const std::int32_t* __restrict__ position,
+                  int used, std::uint8_t* __restrict__ out, unsigned warps) {
   GridLaunchDependents();
-  // (the index arithmetic runs beside the tail of the kernel before, not after it)
-  const std::int64_t i = (static_cast<std::int64_t>(blockIdx.x) * 256) + threadIdx.x;
-  const bool live = i < lanes_total;
-  const std::int64_t group = (live ? i : 0) / 8;  // (col, k / 32)
-  const int part = static_cast<int>(i % 8);
-  const int groups = k / 32;
-  const std::int64_t col = group / groups;
-  const int g = static_cast<int>(group - (col * groups));
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const unsigned chunks = (static_cast<unsigned>(k) + 255u) / 256u;
+  const unsigned warp = (blockIdx.x * 8u) + (threadIdx.x >> 5);
+  const int at_k = static_cast<int>(((warp % chunks) * 256u) + (static_cast<unsigned>(lane) * 8u));
+  const int col0 = static_cast<int>(warp / chunks) * kCols;
+  const bool live = warp < warps && at_k < k;
+  const std::int64_t out_cols = kSlots ? static_cast<std::int64_t>(cols) * used : cols;
   GridDependencyWait();
-  float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  if (live) {
-    const std::int64_t src_row = ids_src != nullptr ? ids_src[col] : col;
-    const std::int64_t at = (src_row * row_stride) + (g * 32) + (part * 4);
-    if constexpr (kBf16) {
-      const uint2 raw = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(x) + at);
-      v[0] = __uint_as_float(raw.x << 16);
-      v[1] = __uint_as_float(raw.x & 0xffff0000u);
-      v[2] = __uint_as_float(raw.y << 16);
-      v[3] = __uint_as_float(raw.y & 0xffff0000u);
+  float v[kCols][8];
+#pragma unroll
+  for (int c = 0; c < kCols; ++c) {
+    const int col = min(col0 + c, cols - 1);
+    if (live) {
+      Load8<kBf16>(x, (static_cast<std::int64_t>(ids_src != nullptr ? ids_src[col] : col) * row_stride) + at_k, v[c]);
     } else {
-      const float4 f = *reinterpret_cast<const float4*>(static_cast<const float*>(x) + at);
-      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[c][i] = 0.0f;
     }
   }
-  float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-  float sum = ((v[0] + v[1]) + v[2]) + v[3];
 #pragma unroll
-  for (int offset = 4; offset > 0; offset >>= 1) {
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, offset));
-    sum = sum + __shfl_xor_sync(0xffffffffu, sum, offset);
-  }
-  if (!live) return;
-  std::uint32_t packed = 0;
-  float d = 0.0f;
-  if (amax > 0.0f) {
-    const float d_inv = 127.0f / amax;
+  for (int c = 0; c < kCols; ++c) {
+    float amax = 0.0f;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int q = static_cast<int>(roundf(v[c] * d_inv));
-      packed |= (static_cast<std::uint32_t>(q) & 0xffu) << (8 * c);
+    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[c][i]));
+    // parts 2j and 2j + 1 of the group's eight (j = lane % 4): parts 4 apart are two lanes apart
+    float even = ((v[c][0] + v[c][1]) + v[c][2]) + v[c][3];
+    float odd = ((v[c][4] + v[c][5]) + v[c][6]) + v[c][7];
+#pragma unroll
+    for (int offset = 2; offset > 0; offset >>= 1) {
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, offset));
+      even = even + __shfl_xor_sync(0xffffffffu, even, offset);
+      odd = odd + __shfl_xor_sync(0xffffffffu, odd, offset);
     }
-    d = 1.0f / d_inv;
-  }
-  std::uint8_t* block = out + ((static_cast<std::int64_t>(g / 4) * cols + col) * 144);
-  *reinterpret_cast<std::uint32_t*>(block + 16 + ((g % 4) * 32) + (part * 4)) = packed;
-  if (part == 0) {
+    const float sum = even + odd;
+    if (!live || col0 + c >= cols) continue;
+    std::uint32_t packed[2] = {0, 0};
+    float d = 0.0f;
+    if (amax > 0.0f) {
+      const float d_inv = 127.0f / amax;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int q = static_cast<int>(roundf(v[c][i] * d_inv));
+        packed[i >> 2] |= (static_cast<std::uint32_t>(q) & 0xffu) << (8 * (i & 3));
+      }
+      d = 1.0f / d_inv;
+    }
     const std::uint32_t ds = static_cast<std::uint32_t>(__half_as_ushort(__float2half_rn(d))) |
-                             (static_cast<std::uint32_t>(__half_as_ushort(__float2half_rn(sum)))
-                              << 16);
-    *reinterpret_cast<std::uint32_t*>(block + ((g % 4) * 4)) = ds;
+                             (static_cast<std::uint32_t>(__half_as_ushort(__float2half_rn(sum))) << 16);
+    const auto store = [&](std::int64_t col) {
+      std::uint8_t* block = out + ((static_cast<std::int64_t>(at_k >> 7) * out_cols) + col) * 144;
+      *reinterpret_cast<uint2*>(block + 16 + (at_k & 127)) = make_uint2(packed[0], packed[1]);
+      if ((lane & 3) == 0) *reinterpret_cast<std::uint32_t*>(block + ((at_k & 127) >> 3)) = ds;
+    };
+    if constexpr (kSlots) {
+      for (int j = 0; j < used; ++j) {
+        const int row = position[(static_cast<std::int64_t>(col0 + c) * used) + j];
+        if (row >= 0) store(row);
+      }
+    } else {
+      store(col0 + c);
+    }
   }
+}
+
+// Four columns a warp where that still fills the chip four times over, else one (203 columns of 2560
+// values would be 510 warps of four).
+template <bool kBf16, bool kSlots>
+int QuantizeMmq(const void* x, std::int64_t row_stride, std::int64_t k, std::int64_t cols,
+                const std::int32_t* ids_src, const std::int32_t* position, int used, void* out, void* stream) {
+  const std::int64_t chunks = (k + 255) / 256;
+  const bool four = ((cols + 3) / 4) * chunks >= static_cast<std::int64_t>(SmCount()) * 32;
+  const std::int64_t warps = chunks * (four ? (cols + 3) / 4 : cols);
+  if (cols > 0x7fffffffLL || k > 0x7fffffffLL || (warps + 7) / 8 > 0x1fffffffLL) {
+    return Reject("mmq.quantize: more blocks than a grid holds");
+  }
+  const auto kernel = four ? &QuantizeMmqKernel<kBf16, 4, kSlots> : &QuantizeMmqKernel<kBf16, 1, kSlots>;
+  const cudaError_t e =
+      LaunchPdl(kernel, dim3(static_cast<unsigned>((warps + 7) / 8)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                x, row_stride, static_cast<int>(k), static_cast<int>(cols), ids_src, position, used,
+                static_cast<std::uint8_t*>(out), static_cast<unsigned>(warps));
+  if (e != cudaSuccess) return Failed(e, "mmq.quantize launch");
+  return 0;
 }
 
 // ------------------------------------------------------------------ slab
@@ -1147,19 +1201,25 @@ int llmp_b200_mmq_quantize(const void* x, int is_bf16, int64_t row_stride, int64
     return Reject("mmq.quantize: input rows and output 16-byte aligned");
   }
   if (const int status = DeviceStatus(); status != 0) return status;
-  const std::int64_t lanes = cols * (k / 32) * 8;
-  const std::int64_t grid = (lanes + 255) / 256;
-  if (grid > 0x7fffffffLL) return Reject("mmq.quantize: more blocks than a grid holds");
-  auto* s = static_cast<cudaStream_t>(stream);
-  const cudaError_t e =
-      is_bf16 ? LaunchPdl(QuantizeMmqKernel<true>, dim3(static_cast<unsigned>(grid)), dim3(256), 0,
-                          s, x, row_stride, static_cast<int>(k), cols, ids_src,
-                          static_cast<std::uint8_t*>(out), lanes)
-              : LaunchPdl(QuantizeMmqKernel<false>, dim3(static_cast<unsigned>(grid)), dim3(256), 0,
-                          s, x, row_stride, static_cast<int>(k), cols, ids_src,
-                          static_cast<std::uint8_t*>(out), lanes);
-  if (e != cudaSuccess) return Failed(e, "mmq.quantize launch");
-  return 0;
+  return is_bf16 ? QuantizeMmq<true, false>(x, row_stride, k, cols, ids_src, nullptr, 0, out, stream)
+                 : QuantizeMmq<false, false>(x, row_stride, k, cols, ids_src, nullptr, 0, out, stream);
+}
+
+int llmp_b200_mmq_quantize_slots(const void* x, int is_bf16, int64_t row_stride, int64_t k, int64_t tokens,
+                                 const int32_t* position, int used, void* out, void* stream) {
+  using namespace llmp_b200;
+  if (x == nullptr || position == nullptr || out == nullptr || k < 128 || k % 128 != 0 || tokens < 1 ||
+      used < 1 || row_stride < k) {
+    return Reject("mmq.quantize_slots: [k, tokens] input with k a positive multiple of 128, [tokens, used] "
+                  "positions");
+  }
+  const int elem = is_bf16 ? 2 : 4;
+  if (!Aligned(x, 16) || (row_stride * elem) % 16 != 0 || !Aligned(out, 16) || !Aligned(position, 4)) {
+    return Reject("mmq.quantize_slots: input rows and output 16-byte aligned, positions 4");
+  }
+  if (const int status = DeviceStatus(); status != 0) return status;
+  return is_bf16 ? QuantizeMmq<true, true>(x, row_stride, k, tokens, nullptr, position, used, out, stream)
+                 : QuantizeMmq<false, true>(x, row_stride, k, tokens, nullptr, position, used, out, stream);
 }
 
 size_t llmp_b200_q4k_slab_bytes(int nrows, int k, int experts) {

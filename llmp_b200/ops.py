@@ -19,7 +19,7 @@ __all__ = ["available", "sm_count", "device_faults", "device_faults_clear", "blo
            "quantize_q8", "vecq", "vecq_ranks", "mmvq", "vecq_f32", "vecq_q8", "vecq_q8_scratch", "vecq_variants", "vecq_block_sums", "mxfp8_padded_rows",
            "mxfp8_quantize", "mxfp8_swizzle", "mxfp8_gemm", "mxfp8_mul_mat_vec", "decode_vector", "decode_rows", "decode_matrix", "decode_grouped", "DECODER_Q8_0", "DECODER_MXFP8_SPLIT",
            "DECODER_MXFP8_ATOMS", "DECODER_BF16", "DECODER_F16", "DECODER_NVFP4_SPLIT", "DECODER_NVFP4_ATOMS",
-           "DECODER_MXFP4_SPLIT", "DECODER_MXFP4_ATOMS", "mmq_quantize", "mmq", "mmq_scratch", "mmq_block_sums", "q4k_relayout", "moe_route", "grouped_gemm",
+           "DECODER_MXFP4_SPLIT", "DECODER_MXFP4_ATOMS", "mmq_quantize", "mmq_quantize_slots", "mmq", "mmq_scratch", "mmq_block_sums", "q4k_relayout", "moe_route", "grouped_gemm",
            "moe_glu_quantize", "moe_combine", "moe_ep_pack", "moe_ffn", "moe_decode", "moe_decode_fits",
            "mmq_glu", "grouped_gemm_glu", "TYPE_Q8_0", "TYPE_Q4_K",
            "TYPE_Q4_0", "TYPE_Q5_0", "TYPE_Q5_K", "TYPE_Q6_K", "TYPE_IQ4_NL",
@@ -379,6 +379,24 @@ def mmq_quantize(x: torch.Tensor, ids_src: torch.Tensor | None = None,
     return out
 
 
+def mmq_quantize_slots(x: torch.Tensor, position: torch.Tensor, used: int) -> torch.Tensor:
+    """x F32 or BF16 [tokens, k] -> Q8_1-MMQ blocks uint8 [k / 128, tokens * used, 144]: token t's
+    blocks in the columns position[t * used + j] (I32, as moe_route leaves it; negative: none), each
+    token quantized once.  A column that no position names is not written."""
+    if not (x.is_cuda and x.dtype in (torch.float32, torch.bfloat16) and x.dim() == 2
+            and x.stride(1) == 1):
+        raise Rejected("mmq_quantize_slots: a CUDA F32 or BF16 [tokens, k] tensor, k contiguous")
+    tokens, k = x.shape
+    _need(position, torch.int32, "mmq_quantize_slots position")
+    if used < 1 or position.numel() != tokens * used or not position.is_contiguous():
+        raise Rejected("mmq_quantize_slots: contiguous I32 [tokens, used] positions")
+    out = torch.empty((max(k // 128, 1), tokens * used, 144), dtype=torch.uint8, device=x.device)
+    N.check(N.lib().llmp_b200_mmq_quantize_slots(
+        x.data_ptr(), int(x.dtype == torch.bfloat16), x.stride(0), k, tokens, position.data_ptr(), used,
+        out.data_ptr(), _stream()), "llmp_b200_mmq_quantize_slots")
+    return out
+
+
 def q4k_relayout(weights: torch.Tensor, k: int, n: int, *, glu: bool = False) -> torch.Tensor:
     """The load-time relayout of Q4_K weights [n, k blocks] or experts [experts, n, k blocks]
     into the tensor core's slab (llmp_b200_q4k_relayout): a uint8 tensor to pass as `slab`.
@@ -699,8 +717,7 @@ def moe_ffn(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, gate_up: 
             moe_combine(y.view(n * used, hidden), None, weights[t0:t1], n, used, out=out[t0:t1])
         return out
     route = moe_route(ids, experts)
-    slots = tokens * used
-    aq = mmq_quantize(x, ids_src=route["token"], cols=slots)
+    aq = mmq_quantize_slots(x[:tokens], route["position"], used)
     if slabs is not None and len(slabs) > 2 and slabs[2] and inter % 128 == 0:
         # slabs[0] interleaves gate and up rows: the GLU and the requantization happen in the
         # gate | up product's write-back (no F32 round trip, no separate pass)

@@ -38,6 +38,33 @@ def test_mmq_activation_blocks_are_bit_exact(cuda, orc, cols, k, bf16):
     assert np.array_equal(got, orc.quantize_mmq_q8_1(x, ids_src=ids))
 
 
+@pytest.mark.parametrize("cols,k,bf16", [(2051, 2432, True), (2050, 2432, False)])
+def test_mmq_activation_blocks_of_many_columns_are_bit_exact(cuda, orc, cols, k, bf16):
+    """Four columns a warp: a last warp of two or three, and a k that is not a multiple of 256."""
+    test_mmq_activation_blocks_are_bit_exact(cuda, orc, cols, k, bf16)
+
+
+@pytest.mark.parametrize("tokens,k,used,bf16", [(1, 128, 1, False), (5, 384, 3, True), (2051, 2432, 2, False)])
+def test_mmq_blocks_of_routed_tokens_are_the_gathered_ones(cuda, orc, tokens, k, used, bf16):
+    """A token quantized once for all its rows: the blocks of the rows gathered and quantized each;
+    a negative position is skipped and a column that no position names stays unwritten."""
+    torch = cuda
+    ops = _ops()
+    rng = np.random.default_rng(tokens + k)
+    x = to_dev(torch, rng.normal(0, 1, size=(tokens, k)).astype(np.float32))
+    if bf16:
+        x = x.bfloat16()
+    position = rng.permutation(tokens * used).astype(np.int32)
+    skipped = position[0]
+    position[0] = -1
+    token = np.zeros(tokens * used, dtype=np.int32)
+    token[position[1:]] = np.arange(1, tokens * used) // used
+    want = ops.mmq_quantize(x, ids_src=to_dev(torch, token))
+    got = ops.mmq_quantize_slots(x, to_dev(torch, position), used)
+    named = [c for c in range(tokens * used) if c != skipped]
+    assert torch.equal(got[:, named], want[:, named])
+
+
 def _check(got, want32, want64, what=""):
     got = got.astype(np.float64)
     assert np.isfinite(got).all(), what

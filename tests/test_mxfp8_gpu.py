@@ -44,6 +44,11 @@ def test_quantizer_codes_and_scales_are_bit_exact(cuda, orc, rows, k, bf16):
     assert np.array_equal(scales.cpu().numpy(), want_scales)
 
 
+def test_quantizer_of_many_rows_is_bit_exact(cuda, orc):
+    """Four rows a warp, a k that is not a multiple of 256, padding rows."""
+    test_quantizer_codes_and_scales_are_bit_exact(cuda, orc, 2051, 2432, True)
+
+
 def test_swizzle_places_scales_in_atoms(cuda, orc):
     torch = cuda
     ops = _ops()
