@@ -9,6 +9,8 @@
 // the grouped GEMM is the Q4_K x Q8_1-MMQ tensor-core kernel of mmq.cu driven
 // by a tile worklist built ON THE DEVICE from the route's offsets (the role
 // of the reference's SetupGroups): nothing waits on the host.
+#include <algorithm>
+
 #include "mmq.cuh"
 #include "tc.cuh"
 
@@ -49,19 +51,22 @@ __host__ Route RouteOf(std::int32_t* base, int experts, int used, int tokens) {
 // llmp_moe.cu:81-160; the blob they leave, moe_layout.h:47-83, is reproduced
 // word for word).  A thread-block cluster of 1 to 8 CTAs, sized by the chunk
 // count, walks four phases separated by cluster barriers:
-//   1. a warp owns whole 64-token chunks.  It clears its chunk's row of
-//      `counts`, then takes the chunk's slots 32 at a time in slot order:
-//      lanes naming the same expert find each other with match.any, the first
-//      of them bumps the chunk's count for that expert (a plain read-modify-
-//      write: the row is the warp's own) and every lane learns its ordinal
-//      within (chunk, expert), parked in position[slot];
-//   2. a thread an expert turns its column of `counts` into the exclusive
-//      prefix over the chunks and leaves the expert's total in offsets[e + 1];
+//   1. a warp owns whole 64-token chunks, neighbouring chunks on different
+//      SMs.  It counts in its own row of shared memory: the chunk's slots 32 at
+//      a time in slot order, lanes naming the same expert find each other with
+//      match.any, the first of them bumps the count and every lane learns its
+//      ordinal within (chunk, expert), parked in position[slot]; then the row
+//      goes to `counts`;
+//   2. a warp an expert turns its column of `counts` into the exclusive prefix
+//      over the chunks, 32 chunks a step, and leaves the total in offsets[e + 1];
 //   3. every CTA scans the totals into its own shared copy of the offsets
 //      (CTA 0 also writes offsets and scale_rows out, after a barrier that
 //      lets the others finish reading the totals);
-//   4. a thread a slot: row = offsets[e] + counts[chunk][e] + ordinal.
-// No atomics, and rows keep token order within an expert by construction.
+//   4. a thread four slots at a time: row = offsets[e] + counts[chunk][e] + ordinal.
+// No atomics, and rows keep token order within an expert by construction.  What bounds it is the
+// round trips to L2, one after another: a batch of loads goes out before the first is used.  (With
+// the counts of phase 1 in global memory, a thread an expert walking the chunks and one slot a thread
+// at a time on as few CTAs as the chunks filled: 64 us for 4096 tokens x 8 of 128 under ncu.)
 constexpr int kRouteThreads = 1024;
 
 __device__ __forceinline__ void ClusterSync() {
@@ -89,9 +94,10 @@ RouteKernel(const std::int32_t* __restrict__ ids, int ids_stride, Route r) {
   const int cta = static_cast<int>(ClusterRank());
   const int gthread = (cta * kRouteThreads) + tid;
   const int gthreads = ctas * kRouteThreads;
-  const int gwarp = gthread >> 5;
+  const int gwarp = ((tid >> 5) * ctas) + cta;  // neighbours on different SMs
   const int gwarps = gthreads >> 5;
   const std::int64_t slots = static_cast<std::int64_t>(r.used) * r.tokens;
+  extern __shared__ int warp_rows[];  // [32 warps][experts]
 
   // Rows no slot reaches read as row 0 of expert 0.
   for (std::int64_t i = gthread; i < slots; i += gthreads) {
@@ -99,52 +105,73 @@ RouteKernel(const std::int32_t* __restrict__ ids, int ids_stride, Route r) {
     r.expert[i] = 0;
   }
   // ---- 1: per-chunk counts and each slot's ordinal within (chunk, expert)
+  constexpr int kBatch = 8;  // ids a lane has on their way
+  int* const row = warp_rows + ((tid >> 5) * r.experts);
   for (int c = gwarp; c < r.chunks; c += gwarps) {
-    std::int32_t* row = r.counts + (static_cast<std::int64_t>(c) * r.experts);
     for (int e = lane; e < r.experts; e += 32) row[e] = 0;
     __syncwarp();
     const int t0 = c * kRouteChunk;
     const int n = (min(t0 + kRouteChunk, r.tokens) - t0) * r.used;
-    for (int i0 = 0; i0 < n; i0 += 32) {
-      const int i = i0 + lane;
-      int e = -1;
-      if (i < n) {
-        e = ids[(static_cast<std::int64_t>(t0 + (i / r.used)) * ids_stride) + (i % r.used)];
-        if (e < 0 || e >= r.experts) e = -1;
+    for (int i0 = 0; i0 < n; i0 += 32 * kBatch) {
+      int ahead[kBatch];
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int i = i0 + (b * 32) + lane;
+        ahead[b] = i < n ? ids[(static_cast<std::int64_t>(t0 + (i / r.used)) * ids_stride) + (i % r.used)] : -1;
       }
-      // lanes without a valid id all fall in the -1 group and write nothing
-      const unsigned same = __match_any_sync(0xffffffffu, e);
-      const int first = __ffs(static_cast<int>(same)) - 1;
-      int seen = 0;
-      if (e >= 0 && lane == first) {
-        seen = row[e];
-        row[e] = seen + __popc(same);
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int i = i0 + (b * 32) + lane;
+        if (i - lane >= n) break;
+        const int e = ahead[b] < 0 || ahead[b] >= r.experts ? -1 : ahead[b];
+        // lanes without a valid id all fall in the -1 group and write nothing
+        const unsigned same = __match_any_sync(0xffffffffu, e);
+        const int first = __ffs(static_cast<int>(same)) - 1;
+        const int seen = e >= 0 ? row[e] : 0;
+        __syncwarp();  // all have read before the leaders write
+        if (e >= 0 && lane == first) row[e] = seen + __popc(same);
+        if (i < n) {
+          r.position[(static_cast<std::int64_t>(t0) * r.used) + i] =
+              e < 0 ? -1 : seen + __popc(same & ((1u << lane) - 1u));
+        }
+        __syncwarp();  // the next 32 read what these wrote
       }
-      seen = __shfl_sync(0xffffffffu, seen, first);
-      if (i < n) {
-        r.position[(static_cast<std::int64_t>(t0) * r.used) + i] =
-            e < 0 ? -1 : seen + __popc(same & ((1u << lane) - 1u));
-      }
-      __syncwarp();  // the next batch's leaders read what this batch's wrote
     }
+    std::int32_t* counts = r.counts + (static_cast<std::int64_t>(c) * r.experts);
+    for (int e = lane; e < r.experts; e += 32) counts[e] = row[e];
+    __syncwarp();
   }
   ClusterSync();
   // ---- 2: counts -> exclusive prefix over the chunks; totals into offsets[e + 1]
-  for (int e = gthread; e < r.experts; e += gthreads) {
-    int running = 0;
-    for (int c = 0; c < r.chunks; ++c) {
-      std::int32_t* at = r.counts + (static_cast<std::int64_t>(c) * r.experts) + e;
-      const int v = *at;
-      *at = running;
-      running += v;
+  for (int e = gwarp; e < r.experts; e += gwarps) {
+    int before = 0;
+    for (int c0 = 0; c0 < r.chunks; c0 += 64) {
+      int count[2];
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const int c = c0 + (b * 32) + lane;
+        count[b] = c < r.chunks ? __ldcg(r.counts + (static_cast<std::int64_t>(c) * r.experts) + e) : 0;
+      }
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const int c = c0 + (b * 32) + lane;
+        int sum = count[b];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const int up = __shfl_up_sync(0xffffffffu, sum, d);
+          if (lane >= d) sum += up;
+        }
+        if (c < r.chunks) r.counts[(static_cast<std::int64_t>(c) * r.experts) + e] = before + sum - count[b];
+        before += __shfl_sync(0xffffffffu, sum, 31);
+      }
     }
-    r.offsets[e + 1] = running;
+    if (lane == 0) r.offsets[e + 1] = before;
   }
   ClusterSync();
   // ---- 3: the offsets (and the rows rounded up to 128 per expert): a block scan
   // of up to 1024 totals, one a thread, kept in shared memory by every CTA.
   {
-    const int total = tid < r.experts ? r.offsets[tid + 1] : 0;
+    const int total = tid < r.experts ? __ldcg(r.offsets + tid + 1) : 0;
     int v[2] = {total, (total + kScaleRows - 1) / kScaleRows * kScaleRows};
 #pragma unroll
     for (int w = 0; w < 2; ++w) {
@@ -187,35 +214,63 @@ RouteKernel(const std::int32_t* __restrict__ ids, int ids_stride, Route r) {
   }
   __syncthreads();
   // ---- 4: each slot's sorted row; each row's token and expert
-  for (std::int64_t slot = gthread; slot < slots; slot += gthreads) {
-    const int ordinal = r.position[slot];
-    if (ordinal < 0) continue;
-    const int t = static_cast<int>(slot / r.used);
-    const int e = ids[(static_cast<std::int64_t>(t) * ids_stride) + (slot % r.used)];
-    const int row = base[e] + r.counts[(static_cast<std::int64_t>(t / kRouteChunk) * r.experts) + e] +
-                    ordinal;
-    r.position[slot] = row;
-    r.token[row] = t;
-    r.expert[row] = e;
+  for (std::int64_t slot0 = gthread; slot0 < slots; slot0 += 4LL * gthreads) {
+    int ordinal[4], e[4], t[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const std::int64_t slot = slot0 + (static_cast<std::int64_t>(b) * gthreads);
+      const bool live = slot < slots;
+      t[b] = live ? static_cast<int>(slot / r.used) : 0;
+      ordinal[b] = live ? __ldcg(r.position + slot) : -1;
+      e[b] = live ? ids[(static_cast<std::int64_t>(t[b]) * ids_stride) + (slot - (static_cast<std::int64_t>(t[b]) * r.used))] : 0;
+    }
+    int earlier[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      earlier[b] = ordinal[b] < 0 ? 0 : __ldcg(r.counts + (static_cast<std::int64_t>(t[b] / kRouteChunk) * r.experts) + e[b]);
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      if (ordinal[b] < 0) continue;
+      const int row = base[e[b]] + earlier[b] + ordinal[b];
+      r.position[slot0 + (static_cast<std::int64_t>(b) * gthreads)] = row;
+      r.token[row] = t[b];
+      r.expert[row] = e[b];
+    }
   }
 }
 
 // The grouped GEMM's tile list from the experts' offsets: entry 0 the count,
 // then (expert, first column) per 128-column tile, experts in order.
-__global__ void BuildTiles(const std::int32_t* __restrict__ offsets, int groups, int capacity,
-                           std::int32_t* __restrict__ worklist) {
+// (One warp's scan; a programmatic dependent of the kernel before, so that the product's launch does
+// not wait for a launch of its own in between.)
+__global__ void __launch_bounds__(256)
+BuildTiles(const std::int32_t* __restrict__ offsets, int groups, int capacity, std::int32_t* __restrict__ worklist) {
   extern __shared__ int first[];  // groups + 1 tile prefix
-  if (threadIdx.x == 0) {
+  GridLaunchDependents();
+  GridDependencyWait();
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  if (threadIdx.x < 32) {
     int running = 0;
-    for (int e = 0; e < groups; ++e) {
-      first[e] = running;
-      running += (offsets[e + 1] - offsets[e] + kMmqTileCols - 1) / kMmqTileCols;
+    for (int e0 = 0; e0 < groups; e0 += 32) {
+      const int e = e0 + lane;
+      int tiles = e < groups ? (offsets[e + 1] - offsets[e] + kMmqTileCols - 1) / kMmqTileCols : 0;
+      const int own = tiles;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, tiles, d);
+        if (lane >= d) tiles += up;
+      }
+      if (e < groups) first[e] = running + tiles - own;
+      running += __shfl_sync(0xffffffffu, tiles, 31);
     }
-    first[groups] = running;
-    worklist[0] = min(running, capacity);
+    if (lane == 0) {
+      first[groups] = running;
+      worklist[0] = min(running, capacity);
+    }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < groups; e += blockDim.x) {
+  for (int e = static_cast<int>(threadIdx.x); e < groups; e += static_cast<int>(blockDim.x)) {
     const int tiles = first[e + 1] - first[e];
     for (int i = 0; i < tiles; ++i) {
       const int at = first[e] + i;
@@ -446,12 +501,22 @@ int llmp_b200_moe_route(const int32_t* ids, int ids_stride, int experts, int use
   if (const int status = DeviceStatus(); status != 0) return status;
   auto* s = static_cast<cudaStream_t>(stream);
   const Route r = RouteOf(out, experts, used, tokens);
-  // A cluster of 1 to 8 CTAs: 32 warps each, a warp a chunk at a time.
-  int ctas = (r.chunks + 31) / 32;
-  ctas = ctas < 1 ? 1 : ctas > 8 ? 8 : ctas;
+  // A cluster of 1 to 8 CTAs, eight chunks a CTA: a chunk is a warp's, and phase 4 wants threads.
+  const int ctas = std::min(8, std::max(1, (r.chunks + 7) / 8));
+  const std::size_t rows = static_cast<std::size_t>(kRouteThreads / 32) * experts * sizeof(int);
+  static thread_local int configured_device = -1;
+  int device = -1;
+  cudaGetDevice(&device);
+  if (configured_device != device) {
+    const cudaError_t allowed = cudaFuncSetAttribute(RouteKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     kRouteThreads / 32 * kMaxExperts * static_cast<int>(sizeof(int)));
+    if (allowed != cudaSuccess) return Failed(allowed, "moe.route attribute");
+    configured_device = device;
+  }
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(static_cast<unsigned>(ctas));
   config.blockDim = dim3(kRouteThreads);
+  config.dynamicSmemBytes = rows;
   config.stream = s;
   cudaLaunchAttribute attribute[1];
   attribute[0].id = cudaLaunchAttributeClusterDimension;
@@ -496,6 +561,11 @@ int llmp_b200_grouped_gemm_glu(const llmp_b200_grouped_gemm_desc* gemm, int glu,
 
 namespace llmp_b200 {
 namespace {
+cudaError_t LaunchTiles(const llmp_b200_grouped_gemm_desc& g, int capacity, std::int32_t* worklist, void* stream) {
+  return LaunchPdl(BuildTiles, dim3(1), dim3(256), (g.groups + 1) * sizeof(int), static_cast<cudaStream_t>(stream),
+                   g.offsets, g.groups, capacity, worklist);
+}
+
 int GroupedGemm(const llmp_b200_grouped_gemm_desc* gemm, const MmqGlu* glu, void* stream) {
   if (gemm == nullptr) return Reject("grouped_gemm: null descriptor");
   const llmp_b200_grouped_gemm_desc& g = *gemm;
@@ -506,9 +576,8 @@ int GroupedGemm(const llmp_b200_grouped_gemm_desc* gemm, const MmqGlu* glu, void
   if (const int status = DeviceStatus(); status != 0) return status;
   const int capacity = TileCapacity(g.groups, g.rows);
   auto* worklist = static_cast<std::int32_t*>(g.scratch);
-  BuildTiles<<<1, 256, (g.groups + 1) * sizeof(int), static_cast<cudaStream_t>(stream)>>>(
-      g.offsets, g.groups, capacity, worklist);
-  if (const int status = Launched("grouped_gemm tile list"); status != 0) return status;
+  const cudaError_t e = LaunchTiles(g, capacity, worklist, stream);
+  if (e != cudaSuccess) return Failed(e, "grouped_gemm tile list");
   const int status = LaunchMmq(MmqOf(g), worklist, capacity, stream, nullptr, glu);
   // The tile list is queued: a refusal now would leave work behind, so report
   // it as a failure after queueing.
@@ -538,9 +607,8 @@ int llmp_b200_grouped_gemm_static(const llmp_b200_grouped_gemm_desc* gemm, int s
   const int capacity = TileCapacity(g.groups, g.rows);
   // BuildTiles rewrites the count and every entry it will hand out, so nothing
   // of an earlier call's list needs clearing.
-  BuildTiles<<<1, 256, (g.groups + 1) * sizeof(int), static_cast<cudaStream_t>(stream)>>>(
-      g.offsets, g.groups, capacity, worklist);
-  if (const int status = Launched("grouped_gemm_static tile list"); status != 0) return status;
+  const cudaError_t e = LaunchTiles(g, capacity, worklist, stream);
+  if (e != cudaSuccess) return Failed(e, "grouped_gemm_static tile list");
   const int status = LaunchMmq(MmqOf(g), worklist, capacity, stream);
   return status > 0 ? -status : status;
 }

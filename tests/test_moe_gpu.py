@@ -37,6 +37,19 @@ def test_route_is_bit_exact(cuda, orc, tokens, experts, used):
     assert (got["token"].cpu().numpy()[valid:] == 0).all()
 
 
+@pytest.mark.parametrize("tokens,experts,used", [(5000, 37, 2), (8200, 1024, 1), (500, 5, 128)])
+def test_route_of_many_chunks_is_bit_exact(cuda, orc, tokens, experts, used):
+    """More than 64 chunks a warp's scan, experts beyond a warp each, several batches of ids a chunk."""
+    torch = cuda
+    ops = _ops()
+    rng = np.random.default_rng(tokens + experts)
+    ids = rng.integers(-1, experts + 1, size=(tokens, used)).astype(np.int32)
+    got = ops.moe_route(to_dev(torch, ids), experts)
+    want = orc.moe_route(ids, experts)
+    for key in ("offsets", "scale_rows", "position", "counts"):
+        assert np.array_equal(got[key].cpu().numpy(), want[key]), key
+
+
 def test_combine_is_bit_exact(cuda, orc):
     torch = cuda
     ops = _ops()
