@@ -31,8 +31,9 @@ cudaError_t LaunchRowMma(const Desc& d, int p, const RowMmaPlan& plan, cudaStrea
   return cudaErrorInvalidValue;
 }
 cudaError_t LaunchRowMmaTokens(const Desc& d, const RowMmaPlan& plan, cudaStream_t stream) {
-  return d.glu != LLMP_B200_GLU_NONE ? LaunchRowMmaTokensOne<true>(d, plan, stream)
-                                     : LaunchRowMmaTokensOne<false>(d, plan, stream);
+  const bool glu = d.glu != LLMP_B200_GLU_NONE;
+  if (d.tokens <= 4) return glu ? LaunchRowMmaTokensOne<4, true>(d, plan, stream) : LaunchRowMmaTokensOne<4, false>(d, plan, stream);
+  return glu ? LaunchRowMmaTokensOne<8, true>(d, plan, stream) : LaunchRowMmaTokensOne<8, false>(d, plan, stream);
 }
 }  // namespace vecq
 }  // namespace llmp_b200

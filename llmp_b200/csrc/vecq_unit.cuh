@@ -73,11 +73,6 @@ __device__ __forceinline__ void StageUnitBlock(unsigned char* acts, TokenActs la
 __device__ __forceinline__ float ProductFloat(int a, int b) {
   return __int_as_float((a * b) + 0x4b400000) - 12582912.0f;
 }
-// Byte `i` of w as a float: 2^23 + it, less 2^23.
-template <int i>
-__device__ __forceinline__ float ByteFloat(std::uint32_t w) {
-  return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u | i)) - 8388608.0f;
-}
 template <int i>
 __device__ __forceinline__ int ByteInt(std::uint32_t w) {
   return static_cast<int>(__byte_perm(w, 0u, 0x4440u | i));
@@ -93,11 +88,6 @@ struct UnitLane {
     codes = acts + (min(g, live - 1) * layout.Pitch()) + (16 * t);
     scales = acts + layout.Scales() + (t * layout.PairPitch());
   }
-};
-
-template <int i>
-struct Index {
-  static constexpr int value = i;
 };
 
 // The rounding of a sum or product that is infinite comes out as inf - inf: a number in its place,

@@ -566,6 +566,42 @@ def test_token_column_rowmma_matches_the_oracle(cuda, orc, variant, n, k, tokens
         ops.vecq(wd, orc.Q4_K, k, n, ops.quantize_q8(to_dev(torch, x[:1])), 1, gate=gd, glu=glu, variant=v)
 
 
+@pytest.mark.parametrize("n,k,tokens,glu,spare", [
+    (2369, 6144, 5, 0, 0),      # a last tile of one row; five tokens in the form of eight
+    (1201, 4608, 3, 1, 0),      # three in the form of four
+    (9000, 2816, 8, 0, 3),      # several passes of rows that lie further apart than their blocks
+    (4097, 5120, 4, 1, 0),      # ... of both matrices
+    (100, 256, 2, 0, 0)])       # one column
+def test_token_columns_at_their_edges(cuda, orc, n, k, tokens, glu, spare):
+    torch = cuda
+    ops = _ops()
+    rng = np.random.default_rng(n + k + tokens)
+    stride = k // 256 + spare
+    v = ops.vecq_variants().index("rowmma.t8")
+    w = synth.q4_k_weights(rng, n, k)
+    g = synth.q4_k_weights(rng, n, k) if glu else None
+    x = rng.normal(0, 1, size=(tokens, k)).astype(np.float32)
+    q8 = ops.quantize_q8(to_dev(torch, x))
+
+    def rows(m):
+        out = np.zeros((n, stride * 144), dtype=np.uint8)
+        out[:, :k // 256 * 144] = m.reshape(n, -1)
+        return to_dev(torch, out)
+    buf = torch.full((tokens * n + 32,), float("nan"), device="cuda")
+    out = buf[: tokens * n].view(tokens, n)
+    ops.vecq(rows(w), orc.Q4_K, k, n, q8, tokens, gate=rows(g) if glu else None, glu=glu, out=out, variant=v,
+             stride_row=stride)
+    torch.cuda.synchronize()
+    assert ops.device_faults() == 0
+    assert torch.isnan(buf[tokens * n:]).all() and torch.isfinite(out).all()
+    if glu:
+        want = orc.vecq(orc.Q4_K, w, q8.cpu().numpy(), k, n, tokens, g=g, glu=glu)[:, 0, :]
+        assert np.abs(out.cpu().numpy() - want).max() <= 4e-5 * np.abs(want).max()
+    else:
+        f32, s64, a64 = orc.vecq(orc.Q4_K, w, q8.cpu().numpy(), k, n, tokens, want64=True)
+        assert_close_to_f64(out.cpu().numpy(), f32[:, 0, :], s64[:, 0, :], a64[:, 0, :], "token columns")
+
+
 def test_rank_table_names_configurations_the_library_has(cuda, orc):
     """Every row of the measured rank table names a launch configuration that exists, and
     the default launch of a listed product gives the oracle's result."""
