@@ -22,6 +22,8 @@
 #include "common.cuh"
 
 namespace llmp_b200 {
+int LaunchQ8_0F32(const llmp_b200_vecq_desc& d, const float* x, std::int64_t x_stride, void* stream);  // vecq.cu
+
 namespace {
 
 using Desc = llmp_b200_mmvq_desc;
@@ -89,6 +91,10 @@ int Run(const Desc& d, bool prepared, int pass, void* stream, int variant = -1) 
   if (d.dst_col_stride > 0x7fffffffLL) return Reject("mmvq: output stride beyond int");
   const void* q8 = d.q8;
   bool queued = false;
+  if (!prepared && d.type == LLMP_B200_TYPE_Q8_0 && variant == -1) {
+    const int status = LaunchQ8_0F32(ProductOf(d, d.scratch, 0, d.cols), d.x, d.x_col_stride, stream);
+    if (status <= 0) return status;
+  }
   if (!prepared) {
     const int status = llmp_b200_q8_1_quantize(d.x, d.k, d.cols, 1, d.x_col_stride, 0, d.scratch,
                                                stream);

@@ -8,6 +8,7 @@
 // load).  The 32-value sum is formed as a butterfly over value indices 16, 8,
 // 4, 2, 1 apart, so the FP16 it rounds to does not depend on the lane layout.
 #include "peer.cuh"
+#include "q8_1.cuh"
 
 namespace llmp_b200 {
 namespace {
@@ -62,34 +63,7 @@ QuantizeQ8_1Kernel(const float* __restrict__ x, std::int64_t k, std::int64_t row
       }
     }
   }
-  float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-  float s[4] = {v[0], v[1], v[2], v[3]};
-#pragma unroll
-  for (int offset = 4; offset > 0; offset >>= 1) {
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, offset));
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      s[c] = s[c] + __shfl_xor_sync(0xffffffffu, s[c], offset);
-    }
-  }
-  const float sum = (s[0] + s[2]) + (s[1] + s[3]);
-  const float d = amax / 127.0f;
-  std::uint32_t packed = 0;
-  if (amax != 0.0f) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int q = static_cast<int>(roundf(v[c] / d));
-      packed |= (static_cast<std::uint32_t>(q) & 0xffu) << (8 * c);
-    }
-  }
-  if (!live) return;
-  *reinterpret_cast<std::uint32_t*>(o + 4 + (lane8 * 4)) = packed;
-  if (lane8 == 0) {
-    const std::uint32_t ds = static_cast<std::uint32_t>(__half_as_ushort(__float2half_rn(d))) |
-                             (static_cast<std::uint32_t>(__half_as_ushort(__float2half_rn(sum)))
-                              << 16);
-    *reinterpret_cast<std::uint32_t*>(o) = ds;
-  }
+  QuantizeQ8_1Lane(v, lane8, live, o);
 }
 
 // The quantizer over a vector that arrives as tagged words (peer.cuh): a thread polls the four

@@ -21,6 +21,7 @@
 #ifndef LLMP_B200_CSRC_VECQ_STREAM_CUH_
 #define LLMP_B200_CSRC_VECQ_STREAM_CUH_
 
+#include "q8_1.cuh"
 #include "vecq_impl.cuh"
 
 namespace llmp_b200 {
@@ -49,6 +50,8 @@ inline RowSplit MakeRowSplit(int nrows, int grid, int warps) {
   s.warp_rem1 = (s.rows_q + 1) % warps;
   return s;
 }
+constexpr int kStreamMaxSmem = 220 * 1024;  // a plan's, the F32 form's activations included
+
 struct StreamPlan {
   int units_per_row;   // UR
   int rows_per_step;   // RS = threads / UR
@@ -63,6 +66,11 @@ struct StreamPlan {
   unsigned int* faults;  // device counter a wait that ran out increments
   RowSplit split;        // the rows of a CTA (the warp part is unused)
   int unit_reciprocal;   // ceil(2^20 / UR): tid / UR without a division (tid < 1024)
+  // Q8_0: F32 activations (rows x_stride apart) that every CTA quantizes itself, into shared memory at
+  // x_at; null: a.y holds the Q8_1 rows.
+  const float* x;
+  long x_stride;
+  int x_at;
 };
 
 __device__ __forceinline__ std::uint32_t SmemAddr(const void* p) {
@@ -407,13 +415,29 @@ VecQStreamKernel(const Desc a, const StreamPlan plan) {
   }
   GridDependencyWait();
 
+  const std::uint8_t* y = static_cast<const std::uint8_t*>(a.y);
+  std::size_t y_token = static_cast<std::size_t>(a.y_token) * 36;
+  if constexpr (Unit::kUnitElems == 128) {
+    if (plan.x != nullptr) {
+      // whole warps: a row's blocks are a multiple of four
+      const int blocks = UR * 4, lane8 = tid & 7;
+      for (int i = tid; i < a.tokens * blocks * 8; i += kStreamThreads) {
+        const int block = i >> 3, t = block / blocks, b = block - (t * blocks);
+        const float4 f = *reinterpret_cast<const float4*>(plan.x + (t * plan.x_stride) + (b * 32) + (lane8 * 4));
+        const float v[4] = {f.x, f.y, f.z, f.w};
+        QuantizeQ8_1Lane(v, lane8, true, smem + plan.x_at + (block * 36));
+      }
+      __syncthreads();
+      y = smem + plan.x_at;
+      y_token = static_cast<std::size_t>(blocks) * 36;
+    }
+  }
   // The thread's activations: unit u of each token's Q8_1 row.
   UnitActs<Unit> acts[P];
 #pragma unroll
   for (int j = 0; j < P; ++j) {
     const int t = min(j, a.tokens - 1);
-    acts[j].Load(static_cast<const std::uint8_t*>(a.y) +
-                     (static_cast<std::size_t>(t) * a.y_token * 36), u);
+    acts[j].Load(y + (t * y_token), u);
   }
 
   bool healthy = true;
@@ -523,6 +547,7 @@ inline bool PlanStream(const Desc& d, int unit_elems, int block_bytes, int block
   plan->packed = d.stride_row == d.ncols_x / block_elems;
   plan->split = MakeRowSplit(d.nrows, plan->grid, 1);
   plan->unit_reciprocal = ((1 << 20) + ur - 1) / ur;
+  plan->x = nullptr;
   plan->faults = FaultCounter();
   return plan->faults != nullptr;
 }
@@ -530,9 +555,15 @@ inline bool PlanStream(const Desc& d, int unit_elems, int block_bytes, int block
 template <typename Unit, int P, bool kGlu>
 cudaError_t LaunchStreamOne(const Desc& d, const StreamPlan& plan, cudaStream_t stream) {
   auto* kernel = VecQStreamKernel<Unit, P, kGlu>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             plan.smem_bytes);
-  if (e != cudaSuccess) return e;
+  // (once a thread and device, for the most that a plan asks for: a call of the runtime less a launch)
+  static thread_local int configured_device = -1;
+  int device = -1;
+  cudaGetDevice(&device);
+  if (configured_device != device) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamMaxSmem);
+    if (e != cudaSuccess) return e;
+    configured_device = device;
+  }
   return LaunchPdl(kernel, dim3(static_cast<unsigned>(plan.grid)), dim3(kStreamThreads),
                    static_cast<std::size_t>(plan.smem_bytes), stream, d, plan);
 }

@@ -34,6 +34,29 @@ def test_mmvq_quantizes_and_multiplies(cuda, orc, wtype, n, k, cols):
     assert ops.device_faults() == 0
 
 
+@pytest.mark.parametrize("n,k,cols,glu", [(1, 128, 1, 0), (2048, 4096, 2, 0), (301, 2560, 3, 1), (64, 2048, 4, 0),
+                                          (64, 2176, 4, 0)])   # the last: more values than one launch takes
+def test_small_q8_0_columns_quantized_in_the_product(cuda, orc, n, k, cols, glu):
+    """One launch for a small Q8_0 product: the bits of the prepared form, also with columns further apart
+    than their values, and with an output that lies over the columns (two launches)."""
+    torch = cuda
+    ops = _ops()
+    rng = np.random.default_rng(n + k)
+    w = to_dev(torch, synth.q8_0_weights(rng, n, k))
+    gate = to_dev(torch, synth.q8_0_weights(rng, n, k)) if glu else None
+    x = torch.zeros((cols, k + 64), device="cuda")
+    x[:, :k] = to_dev(torch, rng.normal(0, 1, size=(cols, k)).astype(np.float32))
+    x[0, 32:64] = 0.0
+    want = ops.mmvq(w, orc.Q8_0, k, n, q8=ops.quantize_q8(x[:, :k].contiguous()), gate=gate, glu=glu)
+    got = ops.mmvq(w, orc.Q8_0, k, n, x[:, :k], gate=gate, glu=glu)
+    assert torch.equal(got, want)
+    if n <= k:
+        over = ops.mmvq(w, orc.Q8_0, k, n, x[:, :k], gate=gate, glu=glu, out=x[:, :n])
+        assert torch.equal(over, want)
+    torch.cuda.synchronize()
+    assert ops.device_faults() == 0
+
+
 def test_mmvq_glu_is_the_fused_product(cuda, orc):
     torch = cuda
     ops = _ops()
