@@ -444,11 +444,16 @@ int llmp_b200_moe_decode(const llmp_b200_moe_decode_desc* desc, void* stream) {
   config.gridDim = dim3(static_cast<unsigned>(SmCount()));
   config.blockDim = dim3(kThreads);
   config.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attribute[1];
-  attribute[0].id = cudaLaunchAttributeCooperative;  // every CTA resident: they meet once
+  // Every CTA resident: they meet once.  A programmatic dependent too: what comes before the dependency
+  // wait touches this CTA's shared memory only, and a layer's launch then runs under the tail of the
+  // one before (one token, 128 experts, top 8, 2048 x 768: 12.5 -> 11.8 us a layer).
+  cudaLaunchAttribute attribute[2];
+  attribute[0].id = cudaLaunchAttributeCooperative;
   attribute[0].val.cooperative = 1;
+  attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
-  config.numAttrs = 1;
+  config.numAttrs = 2;
   const int polls = 1 << 22;  // x 40 ns: a barrier that never fills gives up after 0.2 s
   const int smem = DecodeSmem(a.hidden, a.used * a.inter);
   static thread_local int configured_device = -1;
