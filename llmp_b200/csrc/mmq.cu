@@ -300,14 +300,18 @@ RelayoutQ4KKernel(const std::uint8_t* __restrict__ w, int n, int k, std::int64_t
 
 // ------------------------------------------------------------------ GEMM
 constexpr int kTileCols = 128;  // tokens: the MMA's M, one TMEM lane each
-constexpr int kTileRows = 128;  // weight rows: the MMA's N, one TMEM column each
+// Weight rows: the MMA's N, one TMEM column each.  128, or 64 where the tiles of 128 leave SMs idle
+// (LaunchMmq): the same sums in the same order.
+constexpr int kTileRows = 128;
 constexpr int kBK = 128;        // K bytes a stage: four 32-value groups
 constexpr int kStages = 3;
 // A TMEM buffer holds a group's integer tile and, beside it, its scale tile; two of them are all
 // 512 columns, so the min terms' sum takes a buffer's turn instead of columns of its own.
-constexpr int kBuffers = 2;
-constexpr int kScaleColumn = kTileRows;
-constexpr int kBufferColumns = 2 * kTileRows;
+template <int kRows>
+constexpr int kBuffers = 256 / kRows;
+constexpr int kMaxBuffers = 4;
+template <int kRows>
+constexpr int kBufferColumns = 2 * kRows;
 constexpr int kWBytes = kTileRows * kBK, kYBytes = kTileCols * kBK;
 // The scale tile's operands, one pair a group: K 16 of which only k = 0 is not zero.  K-major
 // without swizzle: 8 rows x 16 bytes (k = 0..7) a core matrix, the groups of 8 rows 128 bytes
@@ -325,6 +329,7 @@ constexpr int kStageBytes = kWBytes + kYBytes + (2 * kStageScaleBytes);
 // raw blocks leave room for one.
 constexpr int kMinTileBytes = 128 * 128;
 constexpr int kMinSteps = 16;  // k-steps a tile of min operands covers
+constexpr double kNarrowWave = 0.68;  // a wave of 64-row tiles against one of 128
 template <bool kSlab>
 constexpr int kMinTiles = kSlab ? 2 : 1;
 // Raw stages: what TMA brings for one super-block column (two k-steps): the 128 weight rows'
@@ -347,8 +352,9 @@ constexpr int kFirstEpilogueWarp = kFirstDecodeWarp + kDecodeWarps;
 // the fold of the one before.
 constexpr int kEpilogueWarps = 8;
 constexpr int kThreads = (kFirstEpilogueWarp + kEpilogueWarps) * 32;
-constexpr int kEpilogueRows = kTileRows / (kEpilogueWarps / 4);  // weight rows a thread
-static_assert(kEpilogueRows == 64, "two 32-row groups a thread");
+template <int kRows>
+constexpr int kEpilogueRows = kRows / (kEpilogueWarps / 4);  // weight rows a thread
+static_assert(kEpilogueRows<kTileRows> == 64, "two 32-row groups a thread");
 template <bool kSlab>
 constexpr int kSmem = (kStages * kStageBytes) + (2 * kMinTiles<kSlab> * kMinTileBytes) +
                       (kRawStages * kRawBytes<kSlab>) + kScaleTileBytes + (2 * kCoreBytes) + 512;
@@ -379,8 +385,8 @@ struct Shared {
   std::uint64_t y_full[kStages];   // the stage's TMA bytes have landed
   std::uint64_t w_full[kStages];   // the decode warps have written their part
   std::uint64_t empty[kStages];    // the tensor core has read the stage
-  std::uint64_t tmem_full[kBuffers];
-  std::uint64_t tmem_empty[kBuffers];
+  std::uint64_t tmem_full[kMaxBuffers];
+  std::uint64_t tmem_empty[kMaxBuffers];
   std::uint64_t raw_full[kRawStages];
   std::uint64_t raw_empty[kRawStages];
   std::uint64_t minw_full[2];  // slab mode: a tile of weight min operands has landed
@@ -426,7 +432,7 @@ __device__ __forceinline__ void PieceWait(std::uint32_t (&c)[16], std::uint32_t 
                : "memory");
 }
 
-template <bool kSlab, bool kSums>
+template <bool kSlab, bool kSums, int kRows>
 __global__ void __launch_bounds__(kThreads, 1)
 MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ CUtensorMap map_w,
              const __grid_constant__ CUtensorMap map_h, const __grid_constant__ CUtensorMap map_mw,
@@ -461,7 +467,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
       tc::MbarInit(&sh->w_full[s], kDecodeWarps);
       tc::MbarInit(&sh->empty[s], 1);
     }
-    for (int b = 0; b < kBuffers; ++b) {
+    for (int b = 0; b < kBuffers<kRows>; ++b) {
       tc::MbarInit(&sh->tmem_full[b], 1);
       tc::MbarInit(&sh->tmem_empty[b], kEpilogueWarps);
     }
@@ -499,7 +505,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
   // against sorted columns [col0, col0 + 128) of that expert's range, row tiles fastest.  With a
   // worklist (built on the device from the expert bounds) column tile y names entry y: {expert,
   // first column}; entry 0 holds the entry count.
-  const int row_tiles = (a.nrows + kTileRows - 1) / kTileRows;
+  const int row_tiles = (a.nrows + kRows - 1) / kRows;
   const int col_tiles = p.worklist != nullptr ? min(p.worklist[0], p.col_tiles) : p.col_tiles;
   const std::int64_t tiles = static_cast<std::int64_t>(row_tiles) * col_tiles *
                              (p.worklist == nullptr && a.expert_bounds != nullptr ? a.experts : 1);
@@ -541,7 +547,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
       for (std::int64_t i = blockIdx.x; i < tiles && ok && !*abort_flag; i += gridDim.x) {
         const Tile tile = tile_at(i);
         if (tile.col0 >= tile.c_end) continue;
-        const int expert = tile.expert, col0 = tile.col0, row0 = tile.row_tile * kTileRows;
+        const int expert = tile.expert, col0 = tile.col0, row0 = tile.row_tile * kRows;
         for (int ks = 0; ks < ksteps; ++ks, ++it) {
           if ((ks & 1) == 0) {
             // One super-block column (k-steps ks, ks + 1): the tokens' block headers and the
@@ -553,11 +559,11 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
               break;
             }
             unsigned char* stage = raw + (rs * kRawBytes<kSlab>);
-            tc::MbarExpectTx(&sh->raw_full[rs], kRawBytes<kSlab>);
+            tc::MbarExpectTx(&sh->raw_full[rs], kSlab ? kRawBytes<kSlab> : kRawBytes<kSlab> - ((kTileRows - kRows) * 144));
             if constexpr (kSlab) {
               // k is a multiple of 256: the two k-steps' tiles are 4 KB in a row
               const float* src = p.ax + ((((static_cast<std::int64_t>(expert) * p.ax_row_tiles) +
-                                           tile.row_tile) * p.ax_ksteps + ks) * 512);
+                                           (tile.row_tile * kRows / kTileRows)) * p.ax_ksteps + ks) * 512);
               tc::BulkLoad(stage, src, 2 * kAxBytes, &sh->raw_full[rs]);
             } else {
               asm volatile(
@@ -585,7 +591,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
                 break;
               }
               ++mins;
-              tc::MbarExpectTx(&sh->minw_full[mt], kMinTileBytes);
+              tc::MbarExpectTx(&sh->minw_full[mt], kRows * 128);
               asm volatile(
                   "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
                   " [%0], [%1, {%3, %4, %5}], [%2];"
@@ -601,7 +607,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
             give_up();
             break;
           }
-          tc::MbarExpectTx(&sh->y_full[s], kSlab ? kYBytes + kWBytes : kYBytes);
+          tc::MbarExpectTx(&sh->y_full[s], kSlab ? kYBytes + (kRows * kBK) : kYBytes);
           asm volatile(
               "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
               " [%0], [%1, {%3, %4, %5}], [%2];"
@@ -650,6 +656,8 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
         }
         const unsigned char* stage = raw + (rs * kRawBytes<kSlab>);
         const int kk = ks % kMinSteps;
+        // a slab's scales come for 128 rows
+        const int ax_row = kSlab ? (tile.row_tile * kRows) % kTileRows : 0;
 #pragma unroll  // the rows of a thread are independent: their latencies overlap
         for (int t = t0; t < kTileRows; t += kDecodeWarps * 32) {
           const int row_at = ((t >> 3) * 128) + ((t & 7) * 16);  // row t of a scale tile
@@ -659,9 +667,11 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
           // the 128-byte row, 16-byte chunks swizzled like the int8 tiles.
           const int at = ((t >> 3) * 1024) + ((t & 7) * 128) + ((((kk >> 1) ^ (t & 7))) * 16) +
                          ((kk & 1) * 8);
-          if constexpr (kSlab) {
+          if (t >= kRows) {
+            // (a tile of 64 rows: the second half of the tokens only)
+          } else if constexpr (kSlab) {
             // (d * sc)_half comes widened to F32: back to half precision, exactly.
-            const float* ax = reinterpret_cast<const float*>(stage + (half * kAxBytes)) + t;
+            const float* ax = reinterpret_cast<const float*>(stage + (half * kAxBytes)) + ax_row + t;
 #pragma unroll
             for (int gl = 0; gl < 4; ++gl) {
               *reinterpret_cast<uint4*>(sw + (gl * kScaleTileBytes)) =
@@ -725,7 +735,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
               const int pk = pad % kMinSteps;
               const int pat = ((t >> 3) * 1024) + ((t & 7) * 128) + ((((pk >> 1) ^ (t & 7))) * 16) +
                               ((pk & 1) * 8);
-              if constexpr (!kSlab) {
+              if (!kSlab && t < kRows) {
                 *reinterpret_cast<uint2*>(min_w + (mt * kMinTileBytes) + pat) = make_uint2(0u, 0u);
               }
               *reinterpret_cast<uint2*>(min_y + (mt * kMinTileBytes) + pat) = make_uint2(0u, 0u);
@@ -749,8 +759,8 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
     const bool elected = tc::ElectOne();
     // A (M, the TMEM lanes): tokens, signed int8.  B (N, the TMEM columns): weight
     // rows, unsigned codes.
-    const std::uint32_t idesc = tc::IdescI8(kTileCols, kTileRows, true, false);
-    const std::uint32_t fdesc = tc::IdescF16(kTileCols, kTileRows);
+    const std::uint32_t idesc = tc::IdescI8(kTileCols, kRows, true, false);
+    const std::uint32_t fdesc = tc::IdescF16(kTileCols, kRows);
     const std::uint64_t one_y = ScaleDesc(cores, zeros, 0), one_w = ScaleDesc(cores + kCoreBytes, zeros, 0);
     std::uint32_t turn = 0, it = 0, mins = 0;  // turn: of the TMEM buffers
     bool ok = true;
@@ -772,20 +782,20 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
         const unsigned char* sy = scale_y + (s * kStageScaleBytes);
 #pragma unroll
         for (int gl = 0; gl < 4; ++gl, ++turn) {
-          const int b = static_cast<int>(turn % kBuffers);
+          const int b = static_cast<int>(turn % kBuffers<kRows>);
           const std::uint64_t swd = ScaleDesc(sw + (gl * kScaleTileBytes), zeros);
           const std::uint64_t syd = ScaleDesc(sy + (gl * kScaleTileBytes), zeros);
-          ok = tc::MbarWait(&sh->tmem_empty[b], ((turn / kBuffers) & 1u) ^ 1u);
+          ok = tc::MbarWait(&sh->tmem_empty[b], ((turn / kBuffers<kRows>) & 1u) ^ 1u);
           if (!__all_sync(0xffffffffu, ok)) {
             ok = false;
             break;
           }
           tc::TcFenceAfter();
           if (elected) {
-            const std::uint32_t d = tmem + (b * kBufferColumns);
+            const std::uint32_t d = tmem + (b * kBufferColumns<kRows>);
             tc::MmaF16(d, one_y, one_w, fdesc, false);
             tc::MmaI8(d, ydesc + (gl * 2), wdesc + (gl * 2), idesc, true);
-            tc::MmaF16(d + kScaleColumn, syd, swd, fdesc, false);
+            tc::MmaF16(d + kRows, syd, swd, fdesc, false);
             tc::TcCommit(&sh->tmem_full[b]);
             if (gl == 3) tc::TcCommit(&sh->empty[s]);
           }
@@ -795,8 +805,8 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
         // each, the operands of four k-steps) into the next buffer.
         if (ks % kMinSteps == kMinSteps - 1 || ks == ksteps - 1) {
           const int mt = static_cast<int>(mins % kMins);
-          const int b = static_cast<int>(turn % kBuffers);
-          ok = tc::MbarWait(&sh->tmem_empty[b], ((turn / kBuffers) & 1u) ^ 1u);
+          const int b = static_cast<int>(turn % kBuffers<kRows>);
+          ok = tc::MbarWait(&sh->tmem_empty[b], ((turn / kBuffers<kRows>) & 1u) ^ 1u);
           if constexpr (kSlab) ok = ok && tc::MbarWait(&sh->minw_full[mt], (mins / kMins) & 1);
           if (!__all_sync(0xffffffffu, ok)) {
             ok = false;
@@ -808,7 +818,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
             const std::uint64_t mwd = tc::SmemDesc(min_w + (mt * kMinTileBytes), true, 1024);
             const int last = (ks % kMinSteps) / 4;
             for (int q = 0; q <= last; ++q) {  // 32 bytes along the swizzled row each
-              tc::MmaF16(tmem + (b * kBufferColumns), myd + (q * 2), mwd + (q * 2), fdesc, q > 0);
+              tc::MmaF16(tmem + (b * kBufferColumns<kRows>), myd + (q * 2), mwd + (q * 2), fdesc, q > 0);
             }
             tc::TcCommit(&sh->tmem_full[b]);
             tc::TcCommit(&sh->min_free[mt]);
@@ -830,8 +840,8 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
     const int rowgroup = ew >> 2;           // which kEpilogueRows weight rows
     const int tt = (quadrant * 32) + lane;  // token of the tile
     const std::uint32_t base =
-        tmem + (static_cast<std::uint32_t>(quadrant * 32) << 16) + (rowgroup * kEpilogueRows);
-    std::uint64_t acc2[kEpilogueRows / 2];  // rows 2i, 2i + 1
+        tmem + (static_cast<std::uint32_t>(quadrant * 32) << 16) + (rowgroup * kEpilogueRows<kRows>);
+    std::uint64_t acc2[kEpilogueRows<kRows> / 2];  // rows 2i, 2i + 1
     std::uint32_t ca[16], sa[16], cb[16], sb[16];  // two pieces
     std::uint32_t turn = 0;
     bool ok = true, ahead = false;  // ahead: the group's first piece is already on its way
@@ -849,7 +859,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
       // verification: the exact group sums, before any float touches them
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        const int row = row0 + (rowgroup * kEpilogueRows) + (piece * 16) + j;
+        const int row = row0 + (rowgroup * kEpilogueRows<kRows>) + (piece * 16) + j;
         if (row < a.nrows) {
           p.sums[((static_cast<std::size_t>(col) * a.nrows + row) * (a.k / 32)) + group] =
               static_cast<std::int32_t>(c[j] - kFloatBits);
@@ -858,26 +868,26 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
     };
     const auto load = [&](std::uint32_t from, std::uint32_t (&c)[16], std::uint32_t (&s)[16]) {
       tc::TmemLoad16(from, c);
-      tc::TmemLoad16(from + kScaleColumn, s);
+      tc::TmemLoad16(from + kRows, s);
     };
     const int groups = ksteps * 4;
     for (std::int64_t i = blockIdx.x; i < tiles && ok && !*abort_flag; i += gridDim.x) {
       const Tile tile = tile_at(i);
       const int c_end = tile.c_end;
       if (tile.col0 >= c_end) continue;
-      const int row0 = tile.row_tile * kTileRows;
+      const int row0 = tile.row_tile * kRows;
       const int col = tile.col0 + tt;  // this thread's sorted column
 #pragma unroll
-      for (int j = 0; j < kEpilogueRows / 2; ++j) acc2[j] = 0ull;
+      for (int j = 0; j < kEpilogueRows<kRows> / 2; ++j) acc2[j] = 0ull;
       // A k-step's four groups a turn of the loop: 4096 tokens x 4096 -> 14336 1320 us with one, 1233
       // with two, 1211 with four, 1347 with eight, whose code misses the instruction cache.  (The min
       // terms take a buffer's turn too, so buffers and parities stay run-time values.)
 #pragma unroll 4
       for (int g = 0; g < groups; ++g) {
-        const int b = static_cast<int>(turn % kBuffers);
-        const std::uint32_t at = base + (b * kBufferColumns);
+        const int b = static_cast<int>(turn % kBuffers<kRows>);
+        const std::uint32_t at = base + (b * kBufferColumns<kRows>);
         if (!ahead) {
-          ok = tc::MbarWait(&sh->tmem_full[b], (turn / kBuffers) & 1u);
+          ok = tc::MbarWait(&sh->tmem_full[b], (turn / kBuffers<kRows>) & 1u);
           if (!__all_sync(0xffffffffu, ok)) {
             ok = false;
             break;
@@ -886,25 +896,23 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
           load(at, ca, sa);
         }
         ++turn;
-        PieceWait(ca, sa);
-        load(at + 16, cb, sb);
-        if constexpr (kSums) {
-          if (col < c_end) check(g, 0, col, row0, ca);
+        constexpr int kPieces = kEpilogueRows<kRows> / 16;
+#pragma unroll
+        for (int piece = 0; piece < kPieces; piece += 2) {
+          PieceWait(ca, sa);
+          load(at + (16 * piece) + 16, cb, sb);
+          if constexpr (kSums) {
+            if (col < c_end) check(g, piece, col, row0, ca);
+          }
+          fold(piece, ca, sa);
+          PieceWait(cb, sb);
+          if (piece + 2 == kPieces) break;
+          load(at + (16 * piece) + 32, ca, sa);
+          if constexpr (kSums) {
+            if (col < c_end) check(g, piece + 1, col, row0, cb);
+          }
+          fold(piece + 1, cb, sb);
         }
-        fold(0, ca, sa);
-        PieceWait(cb, sb);
-        load(at + 32, ca, sa);
-        if constexpr (kSums) {
-          if (col < c_end) check(g, 1, col, row0, cb);
-        }
-        fold(1, cb, sb);
-        PieceWait(ca, sa);
-        load(at + 48, cb, sb);
-        if constexpr (kSums) {
-          if (col < c_end) check(g, 2, col, row0, ca);
-        }
-        fold(2, ca, sa);
-        PieceWait(cb, sb);
         // The buffer goes back to the tensor core; the next group's first piece, if it is there
         // already, is requested under this one's last fold.
         tc::TcFenceBefore();
@@ -913,21 +921,21 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
         const bool tail = (g & 63) == 63 || g == groups - 1;
         ahead = false;
         if (!tail) {
-          const int nb = static_cast<int>(turn % kBuffers);
-          ahead = __all_sync(0xffffffffu, tc::MbarTest(&sh->tmem_full[nb], (turn / kBuffers) & 1u));
+          const int nb = static_cast<int>(turn % kBuffers<kRows>);
+          ahead = __all_sync(0xffffffffu, tc::MbarTest(&sh->tmem_full[nb], (turn / kBuffers<kRows>) & 1u));
           if (ahead) {
             tc::TcFenceAfter();
-            load(base + (nb * kBufferColumns), ca, sa);
+            load(base + (nb * kBufferColumns<kRows>), ca, sa);
           }
         }
         if constexpr (kSums) {
-          if (col < c_end) check(g, 3, col, row0, cb);
+          if (col < c_end) check(g, kPieces - 1, col, row0, cb);
         }
-        fold(3, cb, sb);
+        fold(kPieces - 1, cb, sb);
         if (tail) {
           // The min terms of 64 groups: sum of (-dmin * m) * s8, taken by the tensor core.
-          const int mb = static_cast<int>(turn % kBuffers);
-          ok = tc::MbarWait(&sh->tmem_full[mb], (turn / kBuffers) & 1u);
+          const int mb = static_cast<int>(turn % kBuffers<kRows>);
+          ok = tc::MbarWait(&sh->tmem_full[mb], (turn / kBuffers<kRows>) & 1u);
           if (!__all_sync(0xffffffffu, ok)) {
             ok = false;
             break;
@@ -935,8 +943,8 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
           tc::TcFenceAfter();
           ++turn;
 #pragma unroll
-          for (int piece = 0; piece < 4; ++piece) {
-            tc::TmemLoad16(base + (mb * kBufferColumns) + (piece * 16), ca);
+          for (int piece = 0; piece < kPieces; ++piece) {
+            tc::TmemLoad16(base + (mb * kBufferColumns<kRows>) + (piece * 16), ca);
             tc::TmemLoadWait16(ca);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -950,11 +958,14 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
         }
       }
       if (!ok && lane == 0) give_up();
-      float acc[kEpilogueRows];
+      float acc[kEpilogueRows<kRows>];
 #pragma unroll
-      for (int i = 0; i < kEpilogueRows / 2; ++i) Unpack2(acc2[i], acc[2 * i], acc[(2 * i) + 1]);
-      const int first = row0 + (rowgroup * kEpilogueRows);
+      for (int i = 0; i < kEpilogueRows<kRows> / 2; ++i) Unpack2(acc2[i], acc[2 * i], acc[(2 * i) + 1]);
+      const int first = row0 + (rowgroup * kEpilogueRows<kRows>);
+      bool stored = false;
+      if constexpr (kRows == kTileRows) {
       if (p.glu_out != nullptr) {
+        stored = true;
         // The thread's 64 rows are twice 16 gate rows then the 16 up rows of the same outputs: one
         // Q8_1-MMQ group of 32 outputs, whose scale and sum are formed exactly as the quantizer
         // kernel does (eight lanes of four values, xor tree 4, 2, 1).
@@ -993,14 +1004,16 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
               static_cast<std::uint32_t>(__half_as_ushort(__float2half_rn(d))) |
               (static_cast<std::uint32_t>(__half_as_ushort(__float2half_rn(sum))) << 16);
         }
-      } else if (ok && col < c_end) {
+      }
+      }
+      if (!stored && ok && col < c_end) {
         const int dst_col = a.ids_dst != nullptr ? a.ids_dst[col] : col;
         float* out = a.dst + (static_cast<std::size_t>(dst_col) * a.dst_col_stride) + first;
         // 256 contiguous bytes a thread: 128-bit stores when the output allows them
         const bool vector = (a.dst_col_stride % 4 == 0) &&
                             (reinterpret_cast<std::uintptr_t>(a.dst) % 16 == 0);
 #pragma unroll  // fully: a dynamic index would put acc[] in local memory
-        for (int v = 0; v < kEpilogueRows / 4; ++v) {
+        for (int v = 0; v < kEpilogueRows<kRows> / 4; ++v) {
           if (vector && first + (4 * v) + 4 <= a.nrows) {
             reinterpret_cast<float4*>(out)[v] =
                 make_float4(acc[4 * v], acc[(4 * v) + 1], acc[(4 * v) + 2], acc[(4 * v) + 3]);
@@ -1111,6 +1124,16 @@ int LaunchMmq(const llmp_b200_mmq_desc& d, const std::int32_t* worklist, int max
   }
   const auto fail = [&](int status) { return (queued && status > 0) ? -status : status; };
   const Slab layout = SlabOf(d.nrows, d.k, experts);
+  // Tiles of 64 weight rows for a dense product whose tiles of 128 leave SMs idle.Half the
+  // rows a tile are 0.68 of its time (203 tokens x 2560 -> 10240, two waves against three of half tiles: 78.0 /
+  // 78.9 us); 60 tokens x 4096 -> 2048 52.7 -> 41.3, 200 x 2560 -> 4096 41.4 -> 32.4.
+  const auto waves = [&](int tile_rows) {
+    const std::int64_t tiles = static_cast<std::int64_t>((d.nrows + tile_rows - 1) / tile_rows) * ((d.ncols + kTileCols - 1) / kTileCols);
+    return (tiles + SmCount() - 1) / SmCount();
+  };
+  const bool narrow = worklist == nullptr && d.expert_bounds == nullptr && sums == nullptr && glu == nullptr &&
+                      kNarrowWave * static_cast<double>(waves(64)) < static_cast<double>(waves(kTileRows));
+  const cuuint32_t box_rows = narrow ? 64 : kTileRows;
   CUtensorMap map_y, map_w, map_h, map_mw;
   if (!Encode3D(&map_y, encode, static_cast<const std::uint8_t*>(d.y) + 16, 128,
                 static_cast<cuuint64_t>(d.ncols), static_cast<cuuint64_t>(d.k / 128), 144,
@@ -1129,11 +1152,11 @@ int LaunchMmq(const llmp_b200_mmq_desc& d, const std::int32_t* worklist, int max
     if (!Encode3D(&map_w, encode, slab + layout.codes, static_cast<cuuint64_t>(d.k),
                   static_cast<cuuint64_t>(d.nrows), static_cast<cuuint64_t>(experts),
                   static_cast<cuuint64_t>(d.k), static_cast<cuuint64_t>(d.k) * d.nrows, kBK,
-                  kTileRows, 1, true, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
+                  box_rows, 1, true, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
         !Encode3D(&map_mw, encode, slab + layout.mw, static_cast<cuuint64_t>(layout.gpad) * 2,
                   static_cast<cuuint64_t>(d.nrows), static_cast<cuuint64_t>(experts),
                   static_cast<cuuint64_t>(layout.gpad) * 2,
-                  static_cast<cuuint64_t>(layout.gpad) * 2 * d.nrows, 128, kTileRows, 1, true,
+                  static_cast<cuuint64_t>(layout.gpad) * 2 * d.nrows, 128, box_rows, 1, true,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B)) {
       return fail(Reject("mmq: the driver refused a tensor map for the weight slab"));
     }
@@ -1144,7 +1167,7 @@ int LaunchMmq(const llmp_b200_mmq_desc& d, const std::int32_t* worklist, int max
                                                 : row_pitch * static_cast<cuuint64_t>(d.nrows);
     if (!Encode3D(&map_w, encode, d.w, static_cast<cuuint64_t>(d.k / 256) * 144,
                   static_cast<cuuint64_t>(d.nrows), static_cast<cuuint64_t>(experts), row_pitch,
-                  expert_pitch, 144, kTileRows, 1, false, CU_TENSOR_MAP_L2_PROMOTION_L2_256B)) {
+                  expert_pitch, 144, box_rows, 1, false, CU_TENSOR_MAP_L2_PROMOTION_L2_256B)) {
       return fail(Reject("mmq: the driver refused a tensor map for the weight blocks"));
     }
     map_mw = map_w;  // unused
@@ -1170,14 +1193,16 @@ int LaunchMmq(const llmp_b200_mmq_desc& d, const std::int32_t* worklist, int max
     const auto allow = [](const void* kernel, int bytes) {
       return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     };
-    cudaError_t e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<false, false>), kSmem<false>);
-    if (e == cudaSuccess) e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<true, false>), kSmem<true>);
-    if (e == cudaSuccess) e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<false, true>), kSmem<false>);
-    if (e == cudaSuccess) e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<true, true>), kSmem<true>);
+    cudaError_t e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<false, false, kTileRows>), kSmem<false>);
+    if (e == cudaSuccess) e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<true, false, kTileRows>), kSmem<true>);
+    if (e == cudaSuccess) e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<false, true, kTileRows>), kSmem<false>);
+    if (e == cudaSuccess) e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<true, true, kTileRows>), kSmem<true>);
+    if (e == cudaSuccess) e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<false, false, 64>), kSmem<false>);
+    if (e == cudaSuccess) e = allow(reinterpret_cast<const void*>(&MmqQ4KKernel<true, false, 64>), kSmem<true>);
     if (e != cudaSuccess) return fail(Failed(e, "mmq attribute"));
     configured_device = device;
   }
-  std::int64_t tiles = (d.nrows + kTileRows - 1) / kTileRows;
+  std::int64_t tiles = (d.nrows + static_cast<int>(box_rows) - 1) / static_cast<int>(box_rows);
   if (worklist != nullptr) {
     if (max_tiles < 1) return fail(Reject("mmq: a worklist needs its capacity"));
     p.col_tiles = max_tiles;
@@ -1193,8 +1218,9 @@ int LaunchMmq(const llmp_b200_mmq_desc& d, const std::int32_t* worklist, int max
   // operands and first groups come in under a tile's write-back.
   const dim3 grid(static_cast<unsigned>(std::min<std::int64_t>(tiles, SmCount())));
   auto* s = static_cast<cudaStream_t>(stream);
-  const auto kernel = slab != nullptr ? (sums != nullptr ? &MmqQ4KKernel<true, true> : &MmqQ4KKernel<true, false>)
-                                      : (sums != nullptr ? &MmqQ4KKernel<false, true> : &MmqQ4KKernel<false, false>);
+  const auto kernel = narrow ? (slab != nullptr ? &MmqQ4KKernel<true, false, 64> : &MmqQ4KKernel<false, false, 64>)
+                      : slab != nullptr ? (sums != nullptr ? &MmqQ4KKernel<true, true, kTileRows> : &MmqQ4KKernel<true, false, kTileRows>)
+                                      : (sums != nullptr ? &MmqQ4KKernel<false, true, kTileRows> : &MmqQ4KKernel<false, false, kTileRows>);
   const cudaError_t e = LaunchPdl(kernel, grid, dim3(kThreads), slab != nullptr ? kSmem<true> : kSmem<false>, s,
                                   map_y, map_w, map_h, map_mw, p);
   if (e != cudaSuccess) return Failed(e, "mmq launch");
