@@ -373,7 +373,7 @@ int LaunchVecQ(int type, const llmp_b200_vecq_desc* desc, int variant, bool f32_
       return Reject("vecq: the token-column rowmma variants take 2 to 8 tokens");
     }
     if (!(dense && q4 && aligned16 && f32_input == false && q8_dst == nullptr &&
-          PlanRowMma(d, token_columns ? 8 : p, SmCount(), &tiles, ctas, token_columns))) {
+          PlanRowMma(d, token_columns ? (d.tokens <= 4 ? 4 : 8) : p, SmCount(), &tiles, ctas, token_columns))) {
       return Reject("vecq: the rowmma variant takes dense Q4_K products of up to 8 tokens");
     }
     if (fan != nullptr) tiles.fan = *fan;

@@ -87,7 +87,7 @@ template <int P, bool kGlu, int kColumns = 0>
 __global__ void __launch_bounds__(RowMmaWarpLimit(P) * 32, 1)
 VecQRowMmaKernel(const Desc a, const RowMmaPlan plan) {
   constexpr bool kTokenColumns = kColumns != 0;
-  static_assert(!kTokenColumns || P == 8, "token columns: the geometry of eight tokens");
+  static_assert(!kTokenColumns || P == kColumns, "token columns: a pass is the form's tokens");
   constexpr int kMats = kGlu ? 2 : 1;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) std::uint64_t full[kRowMmaMaxTiles];
@@ -426,7 +426,7 @@ inline bool PlanRowMma(const Desc& d, int p, int sms, RowMmaPlan* plan, int ctas
   // A pitch that spreads rows g = 0..7 over the banks for 64-bit loads: 32 or 96 mod 128.
   const bool good = (row_bytes % 128 == 32) || (row_bytes % 128 == 96);
   const int pitch = (contiguous && good) ? row_bytes : ((row_bytes + 127) / 128 * 128) + 32;
-  const int acts_bytes = token_columns ? ColumnActs<8>(ur).Bytes() : (ur * 256) + (ur * 8 * 8);
+  const int acts_bytes = token_columns ? (p == 4 ? ColumnActs<4>(ur).Bytes() : ColumnActs<8>(ur).Bytes()) : (ur * 256) + (ur * 8 * 8);
   const int all_acts = token_columns ? acts_bytes : p * acts_bytes;
   const int budget = (218 * 1024 / ctas_per_sm) - all_acts - 2048;
   if (budget <= 0) return false;
@@ -495,7 +495,7 @@ cudaError_t LaunchRowMmaOne(const Desc& d, const RowMmaPlan& plan, cudaStream_t 
 
 template <int kColumns, bool kGlu>
 cudaError_t LaunchRowMmaTokensOne(const Desc& d, const RowMmaPlan& plan, cudaStream_t stream) {
-  auto* kernel = VecQRowMmaKernel<8, kGlu, kColumns>;
+  auto* kernel = VecQRowMmaKernel<kColumns, kGlu, kColumns>;
   static thread_local int configured_device = -1;
   int device = -1;
   cudaGetDevice(&device);
