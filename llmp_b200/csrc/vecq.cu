@@ -310,18 +310,28 @@ int LaunchVecQ(int type, const llmp_b200_vecq_desc* desc, int variant, bool f32_
       }
       break;
     }
-    // A product that the table does not have: the row-lane kernel's dot products go up with the
-    // passes' token count (2, 4, 8), the token-column MMAs' time hardly with it.  From five tokens
-    // those, two CTAs an SM for a GLU where they fit (us at 5 and 8 tokens, row-lane first: gate |
-    // up 1280 -> 3072 21.3, 22.1 against 5.5, 6.0; 3328 -> 6400 22.1, 23.0 / 14.1, 14.5; 4608 ->
-    // 9216, one CTA an SM, 36.3, 37.0 / 23.9, 24.4; down 3072 -> 1280 11.1, 12.1 / 4.7, 5.2; 9216 ->
-    // 4608 19.8, 20.9 / 12.5, 12.9), and for a GLU over short rows from three (at 3 tokens 1024 ->
-    // 4096 8.9 against 5.1, 1792 -> 13312 18.9 / 13.7; but 2304 -> 7680 11.3 / 11.6).  The line by k
-    // is on the safe side: with few rows a CTA they win at three and four tokens too (3072 -> 1280
-    // 6.4 against 4.3, gate | up 2048 -> 3584 8.0 / 6.2, 3840 -> 2048 8.6 / 6.7), with many hardly
-    // (9216 -> 4608 12.2 / 12.0); such products stay on row-lane.
-    if (!ranked && d.tokens >= (glu && d.ncols_x < kTokenColumnsShortRow ? 3 : 5)) {
-      for (int v = kTokenColumnsVariant + (glu ? 1 : 0); v >= kTokenColumnsVariant; --v) {
+    // A product that the table does not have: the row-lane kernel's dot products go up with the passes'
+    // token count (2, 4, 8), the token-column MMAs' hardly with it (us with the quantizer, row-lane first).
+    //   Five tokens and more: the MMAs (3840 -> 3840 at 8 12.9 against 6.9, gate | up 2560 -> 7680 25.1 / 12.0).
+    //   Three and four: all but the largest (12288 -> 2560 at 4 13.7 / 11.4, 8192 -> 8192 16.8 / 14.3, but
+    //   14336 -> 5120 20.8 / 21.2), a GLU's large ones only with rows back to back (4608 -> 9216 20.1 / 17.3,
+    //   but 5120 -> 8192 20.1 / 24.3).
+    //   Two: the small ones (8192 -> 2048 8.5 / 5.7, 5120 -> 3072 8.0 / 6.0, but 9216 -> 4608 10.5 / 12.1; gate |
+    //   up 1280 -> 3072 6.1 / 5.2, but 2560 -> 7680 9.2 / 9.3, 3840 -> 5120 9.9 / 10.2).
+    // A GLU of up to 2^24 weights a matrix with two CTAs an SM (2048 -> 6144 at 3 8.2 with one, 7.2 with two;
+    // 1536 -> 12288 9.8 / 10.7).  Products of 1280 rows and fewer stay on row-lane up to four tokens (a GLU
+    // over rows below 2048 values: two): the MMAs would win there too (3072 -> 1280 at 4 8.8 / 4.4), but their
+    // results are stated to be the row-lane kernel's, bit for bit.
+    if (!ranked && d.tokens >= 2) {
+      const std::int64_t weights = static_cast<std::int64_t>(d.ncols_x) * d.nrows;  // of a matrix
+      RowMmaPlan one{};
+      const bool back_to_back = glu && d.tokens <= 4 && PlanRowMma(d, 4, SmCount(), &one, 1, true) && one.packed != 0;
+      bool take = d.tokens >= 5 || (d.tokens >= 3 && glu && d.ncols_x < kTokenColumnsShortRow);
+      if (!take && d.nrows > kTokenColumnsFewRows) {
+        take = d.tokens == 2 ? weights <= (glu ? 1 << 22 : 1 << 24)
+                             : weights <= (glu && !back_to_back ? 1 << 25 : 1 << 26);
+      }
+      for (int v = kTokenColumnsVariant + (glu && weights <= 1 << 24 ? 1 : 0); take && v >= kTokenColumnsVariant; --v) {
         const int status = LaunchVecQ(type, desc, v, false, nullptr, nullptr, nullptr, stream, fan);
         if (status <= 0) return status;
       }

@@ -538,6 +538,7 @@ constexpr int kStreamVariant = kVariantCount - 15;
 constexpr int kRowLaneVariant = kVariantCount - 14;  // and its seven forced forms after it
 constexpr int kTokenColumnsVariant = kVariantCount - 2;  // and its form of two CTAs an SM after it
 constexpr int kTokenColumnsShortRow = 2048;
+constexpr int kTokenColumnsFewRows = 1280;
 constexpr int kRowMmaVariant = kVariantCount - 6;    // its three split forms and the two token-column forms after it
 
 template <typename Unit, int P, int LPR, int R, int U, bool kGlu>
