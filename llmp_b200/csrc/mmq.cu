@@ -329,7 +329,6 @@ constexpr int kStageBytes = kWBytes + kYBytes + (2 * kStageScaleBytes);
 // raw blocks leave room for one.
 constexpr int kMinTileBytes = 128 * 128;
 constexpr int kMinSteps = 16;  // k-steps a tile of min operands covers
-constexpr double kNarrowWave = 0.68;  // a wave of 64-row tiles against one of 128
 template <bool kSlab>
 constexpr int kMinTiles = kSlab ? 2 : 1;
 // Raw stages: what TMA brings for one super-block column (two k-steps): the 128 weight rows'
@@ -1124,15 +1123,12 @@ int LaunchMmq(const llmp_b200_mmq_desc& d, const std::int32_t* worklist, int max
   }
   const auto fail = [&](int status) { return (queued && status > 0) ? -status : status; };
   const Slab layout = SlabOf(d.nrows, d.k, experts);
-  // Tiles of 64 weight rows for a dense product whose tiles of 128 leave SMs idle.Half the
-  // rows a tile are 0.68 of its time (203 tokens x 2560 -> 10240, two waves against three of half tiles: 78.0 /
-  // 78.9 us); 60 tokens x 4096 -> 2048 52.7 -> 41.3, 200 x 2560 -> 4096 41.4 -> 32.4.
-  const auto waves = [&](int tile_rows) {
-    const std::int64_t tiles = static_cast<std::int64_t>((d.nrows + tile_rows - 1) / tile_rows) * ((d.ncols + kTileCols - 1) / kTileCols);
-    return (tiles + SmCount() - 1) / SmCount();
-  };
+  // Tiles of 64 weight rows for a dense product whose tiles of 64 all run at once: a tile is 0.68 of
+  // the time of one of 128, so they pay where twice as many are still one wave (60 tokens x 4096 -> 2048
+  // 52.7 -> 41.3 us, 200 x 2560 -> 4096 41.4 -> 32.4; three waves against two, 203 x 2560 -> 10240: 78.9 / 78.0).
+  const std::int64_t half_tiles = static_cast<std::int64_t>((d.nrows + 63) / 64) * ((d.ncols + kTileCols - 1) / kTileCols);
   const bool narrow = worklist == nullptr && d.expert_bounds == nullptr && sums == nullptr && glu == nullptr &&
-                      kNarrowWave * static_cast<double>(waves(64)) < static_cast<double>(waves(kTileRows));
+                      half_tiles <= SmCount();
   const cuuint32_t box_rows = narrow ? 64 : kTileRows;
   CUtensorMap map_y, map_w, map_h, map_mw;
   if (!Encode3D(&map_y, encode, static_cast<const std::uint8_t*>(d.y) + 16, 128,
