@@ -66,7 +66,8 @@ __host__ Route RouteOf(std::int32_t* base, int experts, int used, int tokens) {
 // No atomics, and rows keep token order within an expert by construction.  What bounds it is the
 // round trips to L2, one after another: a batch of loads goes out before the first is used.  (With
 // the counts of phase 1 in global memory, a thread an expert walking the chunks and one slot a thread
-// at a time on as few CTAs as the chunks filled: 64 us for 4096 tokens x 8 of 128 under ncu.)
+// at a time on as few CTAs as the chunks filled: 64 us for 4096 tokens x 8 of 128 under ncu; with each
+// token quantized once as well, the block of 128 experts, 2048 x 768, 1412 -> 1313 us.)
 constexpr int kRouteThreads = 1024;
 
 __device__ __forceinline__ void ClusterSync() {

@@ -62,7 +62,7 @@ __device__ __forceinline__ std::uint32_t Pack4(float a, float b, float c, float 
 // A warp takes 256 values of kRows rows, a lane eight of a 32-value block: 16- or 32-byte loads, all
 // rows' on their way together; padding rows (up to the scale atoms) write zero scales.  (A thread four
 // values of one row, with a 64-bit division each, was bound by its instructions: 2048 x 4096 BF16 values
-// 13 us under ncu, 1.9 TB/s.)
+// 13 us under ncu, 1.9 TB/s; the layer 4096 -> 12288 107.9 -> 103.5 us with this form.)
 template <bool kBf16, int kRows>
 __global__ void __launch_bounds__(256)
 QuantizeKernel(const void* __restrict__ x, std::int64_t x_stride, std::uint8_t* __restrict__ codes,
