@@ -76,13 +76,11 @@ __device__ __forceinline__ void MmaU8S8(int (&c)[4], std::uint32_t a0, std::uint
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// kTokenColumns (P == 8): the MMA's eight columns are the TOKENS, not the sub-blocks.  One MMA
-// a sub-block takes all (up to eight) tokens at once - eight MMAs a super-block whatever the
-// token count, against eight a token - and the fragment hands lane (g, t) the sums of rows g
-// and g + 8 for tokens 2t and 2t + 1: it folds all eight sub-blocks itself, in order, and no
-// lanes have to meet.  (A token's F32 bits then differ from the one-token kernels': the order
-// of the sub-blocks' terms is another.)
-// kColumns: the form of the unit, 4 or 8 tokens (0: sub-block columns).
+// kColumns: 0, the sub-blocks' columns; 4 or 8, token columns (vecq_columns.cuh): the MMA's columns
+// are the TOKENS, up to four with the chunk's two sub-blocks or up to eight, P of them a pass - eight
+// MMAs a super-block whatever the token count, against eight a token - and a lane folds all eight
+// sub-blocks of its rows and tokens itself: no lanes have to meet.  (A token's F32 bits then differ
+// from the one-token kernels': the order of the sub-blocks' terms is another.)
 template <int P, bool kGlu, int kColumns = 0>
 __global__ void __launch_bounds__(RowMmaWarpLimit(P) * 32, 1)
 VecQRowMmaKernel(const Desc a, const RowMmaPlan plan) {
