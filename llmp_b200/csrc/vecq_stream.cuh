@@ -415,8 +415,10 @@ VecQStreamKernel(const Desc a, const StreamPlan plan) {
   }
   GridDependencyWait();
 
-  const std::uint8_t* y = static_cast<const std::uint8_t*>(a.y);
-  std::size_t y_token = static_cast<std::size_t>(a.y_token) * 36;
+  // The thread's activations: unit u of each token's Q8_1 row.  (Two loops, not one over a pointer that
+  // may be shared or global: its loads would be generic ones.)
+  UnitActs<Unit> acts[P];
+  bool quantized = false;
   if constexpr (Unit::kUnitElems == 128) {
     if (plan.x != nullptr) {
       // whole warps: a row's blocks are a multiple of four
@@ -428,16 +430,18 @@ VecQStreamKernel(const Desc a, const StreamPlan plan) {
         QuantizeQ8_1Lane(v, lane8, true, smem + plan.x_at + (block * 36));
       }
       __syncthreads();
-      y = smem + plan.x_at;
-      y_token = static_cast<std::size_t>(blocks) * 36;
+#pragma unroll
+      for (int j = 0; j < P; ++j) acts[j].Load(smem + plan.x_at + (min(j, a.tokens - 1) * blocks * 36), u);
+      quantized = true;
     }
   }
-  // The thread's activations: unit u of each token's Q8_1 row.
-  UnitActs<Unit> acts[P];
+  if (!quantized) {
 #pragma unroll
-  for (int j = 0; j < P; ++j) {
-    const int t = min(j, a.tokens - 1);
-    acts[j].Load(y + (t * y_token), u);
+    for (int j = 0; j < P; ++j) {
+      const int t = min(j, a.tokens - 1);
+      acts[j].Load(static_cast<const std::uint8_t*>(a.y) +
+                       (static_cast<std::size_t>(t) * a.y_token * 36), u);
+    }
   }
 
   bool healthy = true;
