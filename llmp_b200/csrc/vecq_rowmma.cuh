@@ -358,11 +358,10 @@ VecQRowMmaKernel(const Desc a, const RowMmaPlan plan) {
       float v[kMats];
       if constexpr (kTokenColumns) {
         // Four chains, a quarter of the roundings in a row: the sums' error stays below the row-lane
-        // kernel's, whose products the launch rule gives to this one (3072 -> 1280 at 8 tokens 9.3e-8
-        // against 9.5e-8 off the double product; one chain 1.0e-7).  Whole fours without a test a
-        // column, and both matrices' sums in one load: with a test each and one matrix after the
-        // other a step of 34 feed-forward blocks took 949 us at 3 tokens and 1066 at 8, and takes 930
-        // and 1055 so (one chain: 939 and 1057); gate | up 2560 -> 10240 at 8 tokens 15.50 -> 15.26.
+        // kernel's, whose products the launch rule gives to this one (3072 -> 1280 at 8 tokens 8.4e-8
+        // against 9.1e-8 off the double product, 5120 -> 3072 at 3 9.2e-8 / 1.0e-7).  Whole fours without a
+        // test a column, and both matrices' sums in one load: with a test each and one matrix after the
+        // other a step of 34 feed-forward blocks took 2 % longer at 3 tokens and 1 % at 8.
         float s[4][kMats] = {};
         const auto add = [&](int chain, int w) {
           if constexpr (kGlu) {
