@@ -193,7 +193,9 @@ typedef struct llmp_b200_mmvq_desc {
 size_t llmp_b200_mmvq_scratch(int k, int cols);
 /* Replaces MulMatVecQ and, with `gate`, MulMatVecQGlu (mul_mat_q.cu:407-416, 502-515): quantize
  * the 1 to 8 columns of x into scratch, then dst[:, c] = W . x[:, c] (or the GLU of the gate and
- * up products).  Two launches: the Q8_1 quantizer and the llmp.vecq product. */
+ * up products).  Two launches, the Q8_1 quantizer and the llmp.vecq product; one for Q8_0 products of
+ * up to 4 columns and 8192 values (k a multiple of 256, dst apart from x).  Either way scratch then holds the columns'
+ * Q8_1 rows, which llmp_b200_mmvq_prepared may share. */
 int llmp_b200_mmvq(const llmp_b200_mmvq_desc* desc, void* stream);
 /* Replaces RunMmvqPrepared (mul_mat_q.cu:431-451): the same product over prepared rows
  * (desc->q8), which another product may share; nothing is quantized, scratch is unused. */

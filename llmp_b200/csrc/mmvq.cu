@@ -8,7 +8,8 @@
 // bytes, mul_mat_q.cu:308-312) and multiplied, or the rows arrive prepared.
 // Here those are thin launchers: the Q8_1 quantizer of q8_1.cu, then the
 // llmp.vecq product (vecq.cu), whose kernels already stream the weights once
-// for every column.
+// for every column.  Of a small Q8_0 product both are one launch (LaunchQ8_0F32),
+// which leaves the rows in scratch all the same.
 //
 // Row invariance.  The reference needs mmvq_rows because GGML's launch geometry,
 // and with it the order a column's sums are added in, changes with the column

@@ -477,8 +477,8 @@ int LaunchVecQ(int type, const llmp_b200_vecq_desc* desc, int variant, bool f32_
 
 // A small Q8_0 product of F32 columns in one launch (MMVQ): the stream kernel's CTAs quantize the columns
 // themselves.  Up to kF32Values values: a CTA's own quantization then takes about what the quantizer's
-// launch did, and the call is a launch shorter (2560 x 256, one column: 15.8 -> 13.3 us).  -> 1: not
-// taken, nothing queued (d.y then is where the caller quantizes to).
+// launch did, and the call is a launch shorter (2560 x 256, one column: 15.8 -> 13.3 us).  d.y: where the
+// Q8_1 rows go, as the quantizer's launch leaves them.  -> 1: not taken, nothing queued.
 int LaunchQ8_0F32(const llmp_b200_vecq_desc& d, const float* x, std::int64_t x_stride, void* stream) {
   constexpr int kF32Values = 8192;
   if (d.tokens > 4 || static_cast<std::int64_t>(d.tokens) * d.ncols_x > kF32Values) return 1;

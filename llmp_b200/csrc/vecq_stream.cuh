@@ -67,7 +67,7 @@ struct StreamPlan {
   RowSplit split;        // the rows of a CTA (the warp part is unused)
   int unit_reciprocal;   // ceil(2^20 / UR): tid / UR without a division (tid < 1024)
   // Q8_0: F32 activations (rows x_stride apart) that every CTA quantizes itself, into shared memory at
-  // x_at; null: a.y holds the Q8_1 rows.
+  // x_at, and that the grid leaves in a.y; null: a.y holds the Q8_1 rows.
   const float* x;
   long x_stride;
   int x_at;
@@ -433,6 +433,16 @@ VecQStreamKernel(const Desc a, const StreamPlan plan) {
 #pragma unroll
       for (int j = 0; j < P; ++j) acts[j].Load(smem + plan.x_at + (min(j, a.tokens - 1) * blocks * 36), u);
       quantized = true;
+      // The rows go to a.y as well, zero blocks up to their ends included: what the quantizer's launch
+      // leaves there.  A share a CTA.
+      const auto* rows = reinterpret_cast<const std::uint32_t*>(smem + plan.x_at);
+      auto* out = static_cast<std::uint32_t*>(const_cast<void*>(a.y));
+      const int words = blocks * 9, row_words = a.y_token * 9;
+      for (int i = (static_cast<int>(blockIdx.x) * kStreamThreads) + tid; i < a.tokens * row_words;
+           i += static_cast<int>(gridDim.x) * kStreamThreads) {
+        const int t = i / row_words, w = i - (t * row_words);
+        out[i] = w < words ? rows[(t * words) + w] : 0u;
+      }
     }
   }
   if (!quantized) {

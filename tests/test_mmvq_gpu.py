@@ -1,6 +1,8 @@
 """GPU parity of the MMVQ entry points (the reference's MulMatVecQ, RunMmvqPrepared,
 MulMatVecQGlu and MulMatVecQRows: src/kernels/ggml/mul_mat_q.cu:407-451, 502-515,
 mmvq_rows.cu:825) against the CPU oracle, through the C ABI."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -53,6 +55,53 @@ def test_small_q8_0_columns_quantized_in_the_product(cuda, orc, n, k, cols, glu)
     if n <= k:
         over = ops.mmvq(w, orc.Q8_0, k, n, x[:, :k], gate=gate, glu=glu, out=x[:, :n])
         assert torch.equal(over, want)
+    torch.cuda.synchronize()
+    assert ops.device_faults() == 0
+
+
+def _kernels_of(torch, queue):
+    """The kernels that queue() launches, counted in a capture of it."""
+    queue()                                        # function attributes are set outside the capture
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        queue()
+    count = C.c_size_t(0)
+    assert C.CDLL("libcuda.so.1").cuGraphGetNodes(C.c_void_p(graph.raw_cuda_graph()), None, C.byref(count)) == 0
+    return count.value
+
+
+@pytest.mark.parametrize("n,k,cols,over,launches", [
+    (256, 2560, 1, False, 1), (1, 256, 1, False, 1),   # rows without padding; half of one padding, one CTA
+    (301, 2304, 3, False, 1), (64, 2048, 4, False, 1),
+    (64, 2304, 4, False, 2), (1, 128, 1, False, 2),    # more values than one launch takes; rows off 16 bytes
+    (64, 256, 2, True, 2)])                            # the output over the columns
+def test_mmvq_leaves_the_columns_rows_in_scratch(cuda, orc, n, k, cols, over, launches):
+    """Whichever launches a Q8_0 call takes, scratch then holds the quantizer's rows, their zero blocks
+    included and nothing past them, for other products to share."""
+    torch = cuda
+    ops = _ops()
+    from llmp_b200 import _native as N
+    rng = np.random.default_rng(n + k + cols)
+    w = to_dev(torch, synth.q8_0_weights(rng, n, k))
+    x = to_dev(torch, rng.normal(0, 1, size=(cols, k)).astype(np.float32))
+    want = ops.quantize_q8(x)
+    rows = want.numel()
+    scratch = torch.full(((rows + 255) // 256 * 256 + 256,), 0xa5, dtype=torch.uint8, device="cuda")
+    out = x[:, :n] if over else torch.empty((cols, n), device="cuda")
+    d = N.MmvqDesc()
+    d.type, d.w, d.k, d.n, d.cols, d.stride_row = orc.Q8_0, w.data_ptr(), k, n, cols, k // 32
+    d.x, d.x_col_stride, d.scratch = x.data_ptr(), x.stride(0), scratch.data_ptr()
+    d.dst, d.dst_col_stride = out.data_ptr(), out.stride(0)
+
+    def queue():
+        N.check(N.lib().llmp_b200_mmvq(C.byref(d), torch.cuda.current_stream().cuda_stream), "mmvq")
+    queue()
+    torch.cuda.synchronize()
+    assert torch.equal(scratch[:rows], want.view(-1))
+    assert (scratch[rows:] == 0xa5).all()
+    shared = ops.mmvq(w, orc.Q8_0, k, n, q8=scratch[:rows].view(cols, -1))
+    assert torch.equal(out, shared)
+    assert _kernels_of(torch, queue) == launches
     torch.cuda.synchronize()
     assert ops.device_faults() == 0
 
