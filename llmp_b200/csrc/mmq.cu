@@ -14,16 +14,18 @@
 // The tensor core, idle for most of it, also forms the group's SCALE products:
 // d8 (per token) x (d*sc)_half (per weight row) is a rank-1 FP16 product (kind::f16, K
 // 16 of which one is not zero, F32 accumulate: 22 bits, exact), written beside the
-// integers; and before them it leaves the bits of 1.5 * 2^23 in the integer tile, another
-// rank-1 product, onto which the integers accumulate: what is loaded is a float that far
-// above the sum.  So the fold is two TMEM loads a piece and a packed subtraction, exact, and
-// a packed multiply-add a pair: acc += C * (d8 * d*sc), one rounding.  (A conversion a value
-// in the subtraction's place, two cycles a warp instruction: 4096 tokens x 4096 -> 14336 1243
-// us against 1227, a routed block of 4096 tokens 1295 / 1265.  The scales by 20 registers a
-// thread, TMEM loads in an MMA fragment's layout and four integer buffers: 1595.  With the scales as
-// broadcast shared-memory loads, two packed instructions a pair and 16 warps of 32
-// rows: 139 warp instructions and 1,030 cycles a group; 2.4e-7 off the double product
-// where this is 2.1e-7.  4096 tokens x 4096 -> 14336: 1.76 ms then, 1.21-1.25 now.)
+// integers, so the fold is two TMEM loads a piece, a conversion a value and one packed
+// multiply-add a pair: acc += C * (d8 * d*sc), one rounding.  Every tile has one MMA kind
+// and shape between two hand-overs: PTX orders two MMAs in flight only where they share the
+// accumulator and the shape.  (So the integers do not accumulate onto the bits of 1.5 * 2^23
+// left by a third rank-1 product, which would spare the conversion, two cycles a warp
+// instruction: 4096 tokens x 4096 -> 14336 1195 us for 1223, a routed block of 4096 tokens 1238
+// for 1304, but nothing says in which order the two kinds would be done, and a commit and a
+// wait between them take 1497 and 1513.  The scales by 20 registers a thread, TMEM loads in an
+// MMA fragment's layout and four integer buffers: 1595.  With the scales as broadcast
+// shared-memory loads, two packed instructions a pair and 16 warps of 32 rows: 139 warp
+// instructions and 1,030 cycles a group; 2.4e-7 off the double product where this is 2.1e-7.
+// 4096 tokens x 4096 -> 14336: 1.76 ms then, 1.22 now.)
 // The MMA's M side (the TMEM lanes) is the TOKENS and its N side (the TMEM columns) the
 // weight rows: a thread's results are contiguous in the output.
 // The min terms need no integer product: sum over groups of (-dmin*m)_half *
@@ -318,11 +320,6 @@ constexpr int kWBytes = kTileRows * kBK, kYBytes = kTileCols * kBK;
 // apart; k = 8..15 of every operand is one shared tile of zeros, reached by the leading offset.
 constexpr int kScaleTileBytes = 128 * 16;
 constexpr int kStageScaleBytes = 4 * kScaleTileBytes;  // [group]
-// Before a group's integers a third rank-1 product, 4096 x 3072, leaves the bits of 1.5 * 2^23 in the
-// tile: the integers accumulate onto them, and what the epilogue loads is a float 12582912 above the
-// sum.  Its operands are a core matrix each, read for every group of eight rows.
-constexpr int kCoreBytes = 8 * 16;
-constexpr std::uint32_t kFloatBits = 0x4b400000u;  // 12582912.0f
 constexpr int kStageBytes = kWBytes + kYBytes + (2 * kStageScaleBytes);
 // The min terms' operands: FP16 [128 rows or tokens][64 groups] K-major, 128-byte
 // swizzled like the int8 tiles; one tile holds 16 k-steps.  With a slab two tiles alternate,
@@ -356,7 +353,7 @@ constexpr int kEpilogueRows = kRows / (kEpilogueWarps / 4);  // weight rows a th
 static_assert(kEpilogueRows<kTileRows> == 64, "two 32-row groups a thread");
 template <bool kSlab>
 constexpr int kSmem = (kStages * kStageBytes) + (2 * kMinTiles<kSlab> * kMinTileBytes) +
-                      (kRawStages * kRawBytes<kSlab>) + kScaleTileBytes + (2 * kCoreBytes) + 512;
+                      (kRawStages * kRawBytes<kSlab>) + kScaleTileBytes + 512;
 static_assert(kSmem<true> <= 232448 && kSmem<false> <= 232448, "a CTA's shared memory");
 
 // Two F32 lanes in one 64-bit register: sm_100's packed F32 arithmetic does two
@@ -410,12 +407,12 @@ struct Params {
   float limit;
 };
 
-// K-major operand without swizzle: 8-row core matrices `sbo` bytes apart, the second half of the
+// K-major operand without swizzle: 8-row core matrices 128 bytes apart, the second half of the
 // K 16 in the tile at `zeros`.
 __device__ __forceinline__ std::uint64_t ScaleDesc(const unsigned char* tile,
-                                                   const unsigned char* zeros, std::uint32_t sbo = 128) {
+                                                   const unsigned char* zeros) {
   const std::uint32_t lbo = (tc::Smem(zeros) - tc::Smem(tile)) >> 4;
-  return tc::SmemDesc(tile, false, sbo) | (static_cast<std::uint64_t>(lbo & 0x3fffu) << 16);
+  return tc::SmemDesc(tile, false, 128) | (static_cast<std::uint64_t>(lbo & 0x3fffu) << 16);
 }
 
 // Both loads of a 16-row piece: the registers of the integers and of the scales are usable only
@@ -445,8 +442,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
   unsigned char* min_y = min_w + (kMins * kMinTileBytes);  // [kMins] tiles: s8 per token
   unsigned char* scale_w = min_y + (kMins * kMinTileBytes);            // [kStages][group] d * sc
   unsigned char* scale_y = scale_w + (kStages * kStageScaleBytes);     // [kStages][group] d8
-  unsigned char* cores = scale_y + (kStages * kStageScaleBytes);       // the two core matrices of the constant
-  unsigned char* zeros = cores + (2 * kCoreBytes);
+  unsigned char* zeros = scale_y + (kStages * kStageScaleBytes);
   unsigned char* raw = zeros + kScaleTileBytes;                        // [kRawStages] raw stages
   Shared* sh = reinterpret_cast<Shared*>(raw + (kRawStages * kRawBytes<kSlab>));
 
@@ -483,9 +479,6 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
   }
   if (threadIdx.x < kScaleTileBytes / 16) {
     reinterpret_cast<uint4*>(zeros)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
-    if (threadIdx.x < 16) {  // rows of (4096, 0, ...) and (3072, 0, ...)
-      reinterpret_cast<uint4*>(cores)[threadIdx.x] = make_uint4(threadIdx.x < 8 ? 0x6c00u : 0x6a00u, 0u, 0u, 0u);
-    }
     tc::FenceProxyAsync();
   }
   if (warp == kMmaWarp) {
@@ -760,7 +753,6 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
     // rows, unsigned codes.
     const std::uint32_t idesc = tc::IdescI8(kTileCols, kRows, true, false);
     const std::uint32_t fdesc = tc::IdescF16(kTileCols, kRows);
-    const std::uint64_t one_y = ScaleDesc(cores, zeros, 0), one_w = ScaleDesc(cores + kCoreBytes, zeros, 0);
     std::uint32_t turn = 0, it = 0, mins = 0;  // turn: of the TMEM buffers
     bool ok = true;
     for (std::int64_t i = blockIdx.x; i < tiles && ok && !*abort_flag; i += gridDim.x) {
@@ -792,8 +784,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
           tc::TcFenceAfter();
           if (elected) {
             const std::uint32_t d = tmem + (b * kBufferColumns<kRows>);
-            tc::MmaF16(d, one_y, one_w, fdesc, false);
-            tc::MmaI8(d, ydesc + (gl * 2), wdesc + (gl * 2), idesc, true);
+            tc::MmaI8(d, ydesc + (gl * 2), wdesc + (gl * 2), idesc, false);
             tc::MmaF16(d + kRows, syd, swd, fdesc, false);
             tc::TcCommit(&sh->tmem_full[b]);
             if (gl == 3) tc::TcCommit(&sh->empty[s]);
@@ -832,8 +823,8 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
   } else {
     // ------------------------------------------------------------ epilogue
     // acc += C * (d8 * d sc) for 64 rows a thread, 16 at a time: a piece is two TMEM loads, the
-    // sums (12582912 above) and the scale products the tensor core formed beside them, and a packed
-    // subtraction and multiply-add a pair.
+    // integers and the scale products the tensor core formed beside them, one conversion a value
+    // and one packed multiply-add a pair.
     const int ew = warp - kFirstEpilogueWarp;
     const int quadrant = warp & 3;          // TMEM lanes this warp may touch
     const int rowgroup = ew >> 2;           // which kEpilogueRows weight rows
@@ -844,12 +835,11 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
     std::uint32_t ca[16], sa[16], cb[16], sb[16];  // two pieces
     std::uint32_t turn = 0;
     bool ok = true, ahead = false;  // ahead: the group's first piece is already on its way
-    const std::uint64_t down = Pack2(-__uint_as_float(kFloatBits), -__uint_as_float(kFloatBits));
     const auto fold = [&](int piece, const std::uint32_t (&c)[16], const std::uint32_t (&s)[16]) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         acc2[(piece * 8) + i] =
-            Fma2(Add2(Pack2(__uint_as_float(c[2 * i]), __uint_as_float(c[(2 * i) + 1])), down),
+            Fma2(Pack2(__int2float_rn(static_cast<int>(c[2 * i])), __int2float_rn(static_cast<int>(c[(2 * i) + 1]))),
                  Pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[(2 * i) + 1])),
                  acc2[(piece * 8) + i]);
       }
@@ -861,7 +851,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
         const int row = row0 + (rowgroup * kEpilogueRows<kRows>) + (piece * 16) + j;
         if (row < a.nrows) {
           p.sums[((static_cast<std::size_t>(col) * a.nrows + row) * (a.k / 32)) + group] =
-              static_cast<std::int32_t>(c[j] - kFloatBits);
+              static_cast<std::int32_t>(c[j]);
         }
       }
     };
@@ -1123,9 +1113,10 @@ int LaunchMmq(const llmp_b200_mmq_desc& d, const std::int32_t* worklist, int max
   }
   const auto fail = [&](int status) { return (queued && status > 0) ? -status : status; };
   const Slab layout = SlabOf(d.nrows, d.k, experts);
-  // Tiles of 64 weight rows for a dense product whose tiles of 64 all run at once: a tile is 0.68 of
-  // the time of one of 128, so they pay where twice as many are still one wave (60 tokens x 4096 -> 2048
-  // 52.7 -> 41.3 us, 200 x 2560 -> 4096 41.4 -> 32.4; three waves against two, 203 x 2560 -> 10240: 78.9 / 78.0).
+  // Tiles of 64 weight rows for a dense product whose tiles of 64 all run at once: a tile is 0.7 to 0.8 of
+  // the time of one of 128, so they pay where twice as many are still one wave (from blocks and from a slab,
+  // 60 tokens x 4096 -> 2048 56.5 -> 40.0 and 49.5 -> 37.4 us, 200 x 2560 -> 4096 40.7 -> 30.9 and 38.0 -> 29.8;
+  // three waves against two, 203 x 2560 -> 10240: 80.7 / 78.3 and 75.5 / 70.3).
   const std::int64_t half_tiles = static_cast<std::int64_t>((d.nrows + 63) / 64) * ((d.ncols + kTileCols - 1) / kTileCols);
   const bool narrow = worklist == nullptr && d.expert_bounds == nullptr && sums == nullptr && glu == nullptr &&
                       half_tiles <= SmCount();
