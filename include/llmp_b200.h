@@ -122,9 +122,12 @@ typedef struct llmp_b200_vecq_desc {
  * variant >= 0: that launch configuration (status > 0 if it does not take the product).
  * variant -1: the configuration that measured fastest on B200 for this very (k, n, GLU,
  * token count) when the rank table has it, else a rule by size: dense Q4_K products of 5 to 8
- * tokens (of 3 to 8 with a GLU and k < 2048) take the token-column kernel, routed Q4_K products of
- * 72 (token, slot) pairs and more the kernel that streams each named expert once, the others
- * variant -2's.  These kernels add a row's super-blocks in different orders, so a token's F32 bits
+ * tokens (of 3 to 8 with a GLU and k < 2048) take the token-column kernel, and so do those of 3 and
+ * 4 tokens and more than 1280 rows in all but the largest sizes (2^26 weights a matrix; 2^25 with a
+ * GLU whose rows are not staged back to back) and of 2 tokens in small ones (2^24; 2^22 with a GLU);
+ * routed Q4_K products of 72 (token, slot) pairs and more take the kernel that streams each named
+ * expert once; the others, dense products of up to 4 tokens and 1280 rows among them (but for the
+ * short-row GLU above), variant -2's.  These kernels add a row's super-blocks in different orders, so a token's F32 bits
  * may differ between token counts and between numbers of pairs (as the reference's MMVQ's do
  * between column counts).
  * variant -2: one kernel for a shape, its geometry the one-token plan's whatever the token

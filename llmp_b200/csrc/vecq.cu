@@ -319,9 +319,9 @@ int LaunchVecQ(int type, const llmp_b200_vecq_desc* desc, int variant, bool f32_
     //   Two: the small ones (8192 -> 2048 8.5 / 5.7, 5120 -> 3072 8.0 / 6.0, but 9216 -> 4608 10.5 / 12.1; gate |
     //   up 1280 -> 3072 6.1 / 5.2, but 2560 -> 7680 9.2 / 9.3, 3840 -> 5120 9.9 / 10.2).
     // A GLU of up to 2^24 weights a matrix with two CTAs an SM (2048 -> 6144 at 3 8.2 with one, 7.2 with two;
-    // 1536 -> 12288 9.8 / 10.7).  Products of 1280 rows and fewer stay on row-lane up to four tokens (a GLU
-    // over rows below 2048 values: two): the MMAs would win there too (3072 -> 1280 at 4 8.8 / 4.4), but their
-    // results are stated to be the row-lane kernel's, bit for bit.
+    // 1536 -> 12288 9.8 / 10.7).  The line at 1280 rows is not where the two sides cross: the MMAs would win
+    // below it too (3072 -> 1280 at 4 8.8 / 4.4), but up to four tokens (a GLU over rows below 2048 values:
+    // two) the declaration of llmp_b200_vecq gives these products variant -2's bits.
     if (!ranked && d.tokens >= 2) {
       const std::int64_t weights = static_cast<std::int64_t>(d.ncols_x) * d.nrows;  // of a matrix
       RowMmaPlan one{};

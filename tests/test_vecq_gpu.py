@@ -212,7 +212,14 @@ def test_routed_experts_match_the_oracle(cuda, orc, tokens, glu):
 @pytest.mark.parametrize("tokens,n,k,glu,same_as", [
     (5, 17, 768, 0, "rowmma.t8"), (8, 1280, 3072, 0, "rowmma.t8"), (4, 1280, 3072, 0, "rowlane"),
     (5, 40, 2304, 1, "rowmma.t8c2"), (4, 40, 2304, 1, "rowlane"), (3, 300, 1792, 1, "rowmma.t8c2"),
-    (2, 300, 1792, 1, "rowlane"), (8, 600, 13312, 0, "rowlane")])   # the last: eight tokens do not fit beside a tile
+    (2, 300, 1792, 1, "rowlane"), (8, 600, 13312, 0, "rowlane"),   # the last: eight tokens do not fit beside a tile
+    # two to four tokens: both sides of each limit of rows and weights
+    (4, 1281, 3072, 0, "rowmma.t8"), (2, 1280, 3072, 0, "rowlane"),
+    (2, 2048, 8192, 0, "rowmma.t8"), (2, 2049, 8192, 0, "rowlane"),
+    (2, 1536, 2560, 1, "rowmma.t8c2"), (2, 1792, 2560, 1, "rowlane"),
+    (4, 8192, 7936, 0, "rowmma.t8"), (3, 5120, 14336, 0, "rowlane"),
+    (3, 5120, 3072, 1, "rowmma.t8c2"), (3, 5632, 3072, 1, "rowmma.t8"),
+    (4, 9216, 4608, 1, "rowmma.t8"), (4, 8192, 5120, 1, "rowlane")])   # rows back to back; rows apart
 def test_products_without_a_rank_row_take_the_rule(cuda, orc, tokens, n, k, glu, same_as):
     """The rule by rows and tokens for products that the rank table does not have: the bits of the
     kernel it names, and the oracle's sums."""
