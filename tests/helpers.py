@@ -1,9 +1,31 @@
 """Shared helpers of the GPU parity tests."""
+import ctypes as C
+
 import numpy as np
 
 
 def to_dev(torch, a):
     return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def captured_grids(torch, queue):
+    """The grid's x of every kernel that queue() launches, from a capture of it."""
+    queue()                                        # function attributes are set outside the capture
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        queue()
+    driver, handle, count = C.CDLL("libcuda.so.1"), C.c_void_p(graph.raw_cuda_graph()), C.c_size_t(0)
+    assert driver.cuGraphGetNodes(handle, None, C.byref(count)) == 0
+    nodes = (C.c_void_p * count.value)()
+    assert driver.cuGraphGetNodes(handle, nodes, C.byref(count)) == 0
+    grids = []
+    for node in nodes:
+        kind, params = C.c_int(-1), (C.c_uint32 * 32)()   # CUDA_KERNEL_NODE_PARAMS: the function, then gridDimX
+        assert driver.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
+        if kind.value == 0:
+            assert driver.cuGraphKernelNodeGetParams(C.c_void_p(node), params) == 0
+            grids.append(params[2])
+    return grids
 
 
 def assert_close_to_f64(got, f32_oracle, sum64, abs64, what=""):

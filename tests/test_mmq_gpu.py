@@ -6,7 +6,7 @@ of the dequantized operands (tests/unit/ggml_ext_ops_test.cc:103-107)."""
 import numpy as np
 import pytest
 
-from helpers import to_dev
+from helpers import captured_grids, to_dev
 from llmp_b200 import synth
 
 pytestmark = pytest.mark.gpu
@@ -147,6 +147,36 @@ def test_ctas_that_take_several_tiles(cuda, orc, cols, n, k, mode):
     assert ops.device_faults() == 0
     want32, want64 = orc.mmq_q4_k(w[-130:], yq.cpu().numpy(), k, 130, want64=True)
     _check(out[:, -130:].cpu().numpy(), want32, want64)
+
+
+@pytest.mark.parametrize("mode", ["raw", "slab"])
+@pytest.mark.parametrize("cols,n,k,row_tiles", [
+    (1, 1, 256, 1), (129, 130, 768, 3),     # a last tile of one row, of two
+    (60, 2048, 1280, 32),                   # whole tiles; a partial section of min terms
+    (200, 4095, 2304, 64),                  # every second tile the far half of a slab's 128 scales; a last row missing
+    (40, 193, 8448, 4),                     # both tiles of min operands reused
+    (60, 9472, 256, 148), (60, 9473, 256, 75)])   # as many tiles of 64 rows as SMs; one more: tiles of 128
+def test_tiles_of_64_rows_give_the_bits_of_tiles_of_128(cuda, orc, cols, n, k, row_tiles, mode):
+    """Small dense products run tiles of 64 weight rows; the group sums' entry and the grouped GEMM of one
+    group always tiles of 128, whose results and exact sums the other tests hold against the oracle."""
+    torch = cuda
+    ops = _ops()
+    assert ops.sm_count() == 148, "the limits above are a B200's"
+    rng = np.random.default_rng(cols + n + k)
+    w = to_dev(torch, synth.q4_k_weights(rng, n, k))
+    yq = ops.mmq_quantize(to_dev(torch, rng.normal(0, 1, size=(cols, k)).astype(np.float32)))
+    slab = ops.q4k_relayout(w, k, n) if mode == "slab" else None
+    wd = None if mode == "slab" else w
+    buf = torch.full((cols * n + 64,), float("nan"), device="cuda")
+    out = buf[: cols * n].view(cols, n)
+    grids = captured_grids(torch, lambda: ops.mmq(wd, yq, k, n, out=out, slab=slab))
+    assert grids == [row_tiles * ((cols + 127) // 128)]
+    offsets = to_dev(torch, np.array([0, cols], dtype=np.int32))
+    assert torch.equal(out, ops.mmq_block_sums(wd, yq, k, n, slab=slab)[0])
+    assert torch.equal(out, ops.grouped_gemm(None if wd is None else wd.view(1, n, -1), yq, offsets, k, n, slab=slab))
+    assert torch.isnan(buf[cols * n:]).all()
+    torch.cuda.synchronize()
+    assert ops.device_faults() == 0
 
 
 def test_routed_mmq_over_expert_sorted_columns(cuda, orc):

@@ -6,7 +6,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from helpers import assert_close_to_f64, to_dev
+from helpers import assert_close_to_f64, captured_grids, to_dev
 from llmp_b200 import synth
 
 pytestmark = pytest.mark.gpu
@@ -59,17 +59,6 @@ def test_small_q8_0_columns_quantized_in_the_product(cuda, orc, n, k, cols, glu)
     assert ops.device_faults() == 0
 
 
-def _kernels_of(torch, queue):
-    """The kernels that queue() launches, counted in a capture of it."""
-    queue()                                        # function attributes are set outside the capture
-    graph = torch.cuda.CUDAGraph(keep_graph=True)
-    with torch.cuda.graph(graph):
-        queue()
-    count = C.c_size_t(0)
-    assert C.CDLL("libcuda.so.1").cuGraphGetNodes(C.c_void_p(graph.raw_cuda_graph()), None, C.byref(count)) == 0
-    return count.value
-
-
 @pytest.mark.parametrize("n,k,cols,over,launches", [
     (256, 2560, 1, False, 1), (1, 256, 1, False, 1),   # rows without padding; half of one padding, one CTA
     (301, 2304, 3, False, 1), (64, 2048, 4, False, 1),
@@ -101,7 +90,7 @@ def test_mmvq_leaves_the_columns_rows_in_scratch(cuda, orc, n, k, cols, over, la
     assert (scratch[rows:] == 0xa5).all()
     shared = ops.mmvq(w, orc.Q8_0, k, n, q8=scratch[:rows].view(cols, -1))
     assert torch.equal(out, shared)
-    assert _kernels_of(torch, queue) == launches
+    assert len(captured_grids(torch, queue)) == launches
     torch.cuda.synchronize()
     assert ops.device_faults() == 0
 
