@@ -951,14 +951,12 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
 #pragma unroll
       for (int i = 0; i < kEpilogueRows<kRows> / 2; ++i) Unpack2(acc2[i], acc[2 * i], acc[(2 * i) + 1]);
       const int first = row0 + (rowgroup * kEpilogueRows<kRows>);
-      bool stored = false;
+      const bool glu = kRows == kTileRows && p.glu_out != nullptr;
       if constexpr (kRows == kTileRows) {
-      if (p.glu_out != nullptr) {
-        stored = true;
         // The thread's 64 rows are twice 16 gate rows then the 16 up rows of the same outputs: one
         // Q8_1-MMQ group of 32 outputs, whose scale and sum are formed exactly as the quantizer
         // kernel does (eight lanes of four values, xor tree 4, 2, 1).
-        if (ok && col < c_end && first < a.nrows) {
+        if (glu && ok && col < c_end && first < a.nrows) {
           float h[32], part[8], amax = 0.0f;
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
@@ -994,8 +992,7 @@ MmqQ4KKernel(const __grid_constant__ CUtensorMap map_y, const __grid_constant__ 
               (static_cast<std::uint32_t>(__half_as_ushort(__float2half_rn(sum))) << 16);
         }
       }
-      }
-      if (!stored && ok && col < c_end) {
+      if (!glu && ok && col < c_end) {
         const int dst_col = a.ids_dst != nullptr ? a.ids_dst[col] : col;
         float* out = a.dst + (static_cast<std::size_t>(dst_col) * a.dst_col_stride) + first;
         // 256 contiguous bytes a thread: 128-bit stores when the output allows them
