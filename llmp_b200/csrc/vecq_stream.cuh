@@ -338,7 +338,9 @@ __device__ __forceinline__ float UnitDot(const Q8_0Unit<4>& w, const UnitActs<Q8
   return v;
 }
 
-template <typename Unit, int P, bool kGlu>
+// kF32: plan.x's columns are quantized here.  (A kernel of its own: with the test at run time the products of
+// prepared rows took up to 4 % longer, 1024 -> 300 at one token 3.25 -> 3.37 us with its quantizer.)
+template <typename Unit, int P, bool kGlu, bool kF32>
 __global__ void __launch_bounds__(kStreamThreads, 1)
 VecQStreamKernel(const Desc a, const StreamPlan plan) {
   constexpr int kMats = kGlu ? 2 : 1;
@@ -415,37 +417,32 @@ VecQStreamKernel(const Desc a, const StreamPlan plan) {
   }
   GridDependencyWait();
 
-  // The thread's activations: unit u of each token's Q8_1 row.  (Two loops, not one over a pointer that
-  // may be shared or global: its loads would be generic ones.)
+  // The thread's activations: unit u of each token's Q8_1 row.
   UnitActs<Unit> acts[P];
-  bool quantized = false;
-  if constexpr (Unit::kUnitElems == 128) {
-    if (plan.x != nullptr) {
-      // whole warps: a row's blocks are a multiple of four
-      const int blocks = UR * 4, lane8 = tid & 7;
-      for (int i = tid; i < a.tokens * blocks * 8; i += kStreamThreads) {
-        const int block = i >> 3, t = block / blocks, b = block - (t * blocks);
-        const float4 f = *reinterpret_cast<const float4*>(plan.x + (t * plan.x_stride) + (b * 32) + (lane8 * 4));
-        const float v[4] = {f.x, f.y, f.z, f.w};
-        QuantizeQ8_1Lane(v, lane8, true, smem + plan.x_at + (block * 36));
-      }
-      __syncthreads();
-#pragma unroll
-      for (int j = 0; j < P; ++j) acts[j].Load(smem + plan.x_at + (min(j, a.tokens - 1) * blocks * 36), u);
-      quantized = true;
-      // The rows go to a.y as well, zero blocks up to their ends included: what the quantizer's launch
-      // leaves there.  A share a CTA.
-      const auto* rows = reinterpret_cast<const std::uint32_t*>(smem + plan.x_at);
-      auto* out = static_cast<std::uint32_t*>(const_cast<void*>(a.y));
-      const int words = blocks * 9, row_words = a.y_token * 9;
-      for (int i = (static_cast<int>(blockIdx.x) * kStreamThreads) + tid; i < a.tokens * row_words;
-           i += static_cast<int>(gridDim.x) * kStreamThreads) {
-        const int t = i / row_words, w = i - (t * row_words);
-        out[i] = w < words ? rows[(t * words) + w] : 0u;
-      }
+  if constexpr (kF32) {
+    static_assert(Unit::kUnitElems == 128, "Q8_0 units of four blocks");
+    // whole warps: a row's blocks are a multiple of four
+    const int blocks = UR * 4, lane8 = tid & 7;
+    for (int i = tid; i < a.tokens * blocks * 8; i += kStreamThreads) {
+      const int block = i >> 3, t = block / blocks, b = block - (t * blocks);
+      const float4 f = *reinterpret_cast<const float4*>(plan.x + (t * plan.x_stride) + (b * 32) + (lane8 * 4));
+      const float v[4] = {f.x, f.y, f.z, f.w};
+      QuantizeQ8_1Lane(v, lane8, true, smem + plan.x_at + (block * 36));
     }
-  }
-  if (!quantized) {
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < P; ++j) acts[j].Load(smem + plan.x_at + (min(j, a.tokens - 1) * blocks * 36), u);
+    // The rows go to a.y as well, zero blocks up to their ends included: what the quantizer's launch
+    // leaves there.  A share a CTA.
+    const auto* rows = reinterpret_cast<const std::uint32_t*>(smem + plan.x_at);
+    auto* out = static_cast<std::uint32_t*>(const_cast<void*>(a.y));
+    const int words = blocks * 9, row_words = a.y_token * 9;
+    for (int i = (static_cast<int>(blockIdx.x) * kStreamThreads) + tid; i < a.tokens * row_words;
+         i += static_cast<int>(gridDim.x) * kStreamThreads) {
+      const int t = i / row_words, w = i - (t * row_words);
+      out[i] = w < words ? rows[(t * words) + w] : 0u;
+    }
+  } else if (active || P > 2) {  // (the test: 1024 -> 300 at one token 3.37 -> 3.27 us, 2048 -> 2048 at four 8.19 -> 8.52)
 #pragma unroll
     for (int j = 0; j < P; ++j) {
       const int t = min(j, a.tokens - 1);
@@ -566,9 +563,12 @@ inline bool PlanStream(const Desc& d, int unit_elems, int block_bytes, int block
   return plan->faults != nullptr;
 }
 
-template <typename Unit, int P, bool kGlu>
+template <typename Unit, int P, bool kGlu, bool kF32 = false>
 cudaError_t LaunchStreamOne(const Desc& d, const StreamPlan& plan, cudaStream_t stream) {
-  auto* kernel = VecQStreamKernel<Unit, P, kGlu>;
+  if constexpr (Unit::kUnitElems == 128 && P <= 4 && !kF32) {
+    if (plan.x != nullptr) return LaunchStreamOne<Unit, P, kGlu, true>(d, plan, stream);
+  }
+  auto* kernel = VecQStreamKernel<Unit, P, kGlu, kF32>;
   // (once a thread and device, for the most that a plan asks for: a call of the runtime less a launch)
   static thread_local int configured_device = -1;
   int device = -1;
