@@ -37,7 +37,7 @@ def test_mmvq_quantizes_and_multiplies(cuda, orc, wtype, n, k, cols):
 
 
 @pytest.mark.parametrize("n,k,cols,glu", [(1, 128, 1, 0), (2048, 4096, 2, 0), (301, 2560, 3, 1), (64, 2048, 4, 0),
-                                          (64, 2176, 4, 0)])   # the last: more values than one launch takes
+                                          (64, 2176, 4, 0), (1, 256, 1, 0)])   # 2176 x 4, k = 128: two launches
 def test_small_q8_0_columns_quantized_in_the_product(cuda, orc, n, k, cols, glu):
     """One launch for a small Q8_0 product: the bits of the prepared form, also with columns further apart
     than their values, and with an output that lies over the columns (two launches)."""
